@@ -127,11 +127,25 @@ __device__ __forceinline__ void bilinear_acc_x2(float q00a, float q00b, float q0
           "f"(fva), "f"(fvb), "f"(wa), "f"(wb));
 }
 
+// The four taps of one voxel: two FP32 samples of the row at shared address a and two of the row
+// at b.
+__device__ __forceinline__ void load_taps(uint32_t a, uint32_t b, float &q00, float &q01, float &q10, float &q11)
+{
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(q00) : "r"(a));
+    asm volatile("ld.shared.f32 %0, [%1+4];" : "=f"(q01) : "r"(a));
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(q10) : "r"(b));
+    asm volatile("ld.shared.f32 %0, [%1+4];" : "=f"(q11) : "r"(b));
+}
+
 // One column's update of the direct kernel over its TZ slices; PACKED walks
-// two slices per step with packed FP32 and gives the same bits.
+// two slices per step with packed FP32 and gives the same bits.  sbase is the
+// 32-bit shared address of the column in the staged box, already offset by
+// -(kMagicBits + box row origin) rows, so a row's address is one IMAD on the
+// bits of the rounded add and the taps beside and below it are an immediate
+// and one add.
 template <int TZ, bool ALL_IN, bool PACKED>
-__device__ __forceinline__ void direct_update(const float *st, uint32_t BW, uint32_t cbase, float fu, float U,
-                                              float U2, float cZ, float Hm1, const float (&aZ)[TZ], float (&acc)[TZ])
+__device__ __forceinline__ void direct_update(uint32_t sbase, uint32_t row_bytes, float fu, float U, float U2,
+                                              float cZ, float Hm1, const float (&aZ)[TZ], float (&acc)[TZ])
 {
     if constexpr (PACKED && (TZ % 2 == 0)) {
 #pragma unroll
@@ -139,15 +153,17 @@ __device__ __forceinline__ void direct_update(const float *st, uint32_t BW, uint
             const float va = slice_v(aZ[z], U, cZ), vb = slice_v(aZ[z + 1], U, cZ);
             float fla, flb, fva, fvb;
             floor_frac_x2(va, vb, fla, flb, fva, fvb);
-            const uint32_t oa = (uint32_t)__float_as_int(fla) * BW + cbase;
-            const uint32_t ob = (uint32_t)__float_as_int(flb) * BW + cbase;
+            const uint32_t oa = (uint32_t)__float_as_int(fla) * row_bytes + sbase;
+            const uint32_t ob = (uint32_t)__float_as_int(flb) * row_bytes + sbase;
             float wa = U2, wb = U2;
             if constexpr (!ALL_IN) {
                 wa = (va >= 0.f && va <= Hm1) ? U2 : 0.f;  // kernel.cu:130-131
                 wb = (vb >= 0.f && vb <= Hm1) ? U2 : 0.f;
             }
-            bilinear_acc_x2(st[oa], st[ob], st[oa + 1], st[ob + 1], st[oa + BW], st[ob + BW], st[oa + BW + 1],
-                            st[ob + BW + 1], fu, fva, fvb, wa, wb, acc[z], acc[z + 1]);
+            float a00, a01, a10, a11, b00, b01, b10, b11;
+            load_taps(oa, oa + row_bytes, a00, a01, a10, a11);
+            load_taps(ob, ob + row_bytes, b00, b01, b10, b11);
+            bilinear_acc_x2(a00, b00, a01, b01, a10, b10, a11, b11, fu, fva, fvb, wa, wb, acc[z], acc[z + 1]);
         }
     } else {
 #pragma unroll
@@ -155,9 +171,9 @@ __device__ __forceinline__ void direct_update(const float *st, uint32_t BW, uint
             const float v = slice_v(aZ[z], U, cZ);
             const float fl = __fadd_rd(v, kMagic);
             const float fv = v - (fl - kMagic);
-            const uint32_t o = (uint32_t)__float_as_int(fl) * BW + cbase;
-            const float q00 = st[o], q01 = st[o + 1];
-            const float q10 = st[o + BW], q11 = st[o + BW + 1];
+            const uint32_t o = (uint32_t)__float_as_int(fl) * row_bytes + sbase;
+            float q00, q01, q10, q11;
+            load_taps(o, o + row_bytes, q00, q01, q10, q11);
             const float top = fmaf(fu, q01 - q00, q00);
             const float bot = fmaf(fu, q11 - q10, q10);
             const float w = ALL_IN ? U2 : ((v >= 0.f && v <= Hm1) ? U2 : 0.f);  // kernel.cu:130-131
@@ -232,11 +248,13 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     for (int z = 0; z < TZ; ++z) acc[z] = 0.f;
 
     const float cZ = P.cZ, Hm1 = P.Hm1;
-    const uint32_t BW = (uint32_t)P.BW;
+    const uint32_t row_bytes = (uint32_t)P.BW * 4u, smem0 = smem_u32(smem);
     int b = 0;
     for (; b < P.N; ++b) {
         const int s = b % STAGES;
         const uint32_t parity = (uint32_t)(b / STAGES) & 1u;
+        float U, u;
+        column_geometry(aX, aY, P.trig[b], P.D, P.cX, U, u);  // before the wait: a divide and the trig load
         const bool got = mbar_wait_bounded(&full[s], parity, kWaitLimitNs);
         if (!got) {
             atomicOr(P.err, ERR_WAIT_TIMEOUT);
@@ -244,8 +262,6 @@ __global__ void __launch_bounds__(TX *TY, MINB)
         }
         const int bx0 = boxo[b].x, by0 = boxo[b].y;
         if (active && got) {
-            float U, u;
-            column_geometry(aX, aY, P.trig[b], P.D, P.cX, U, u);
             if (u >= 0.f && u <= P.Wm1) {  // column inside the detector (kernel.cu:127-128)
                 const float U2 = __fmul_rn(U, U);
                 const float fla = __fadd_rd(u, kMagic);
@@ -256,13 +272,13 @@ __global__ void __launch_bounds__(TX *TY, MINB)
                 const float vlo = fminf(vA, vB), vhi = fmaxf(vA, vB);
                 const int rlo = (int)floorf(vlo) - by0, rhi = (int)floorf(vhi) + 1 - by0;
                 if (col >= 0 && col + 1 < P.BW && rlo >= 0 && rhi < P.BH) {
-                    const uint32_t cbase = (uint32_t)col - (uint32_t)(kMagicBits + by0) * BW;
+                    const uint32_t sbase = smem0 + ((uint32_t)s * P.stage_elems + (uint32_t)col) * 4u -
+                                           (uint32_t)(kMagicBits + by0) * row_bytes;
                     const bool all_in = (vlo >= 0.f) && (vhi <= Hm1);
-                    const float *st = reinterpret_cast<const float *>(stages) + (size_t)s * P.stage_elems;
                     if (all_in)
-                        direct_update<TZ, true, PACKED>(st, BW, cbase, fu, U, U2, cZ, Hm1, aZ, acc);
+                        direct_update<TZ, true, PACKED>(sbase, row_bytes, fu, U, U2, cZ, Hm1, aZ, acc);
                     else
-                        direct_update<TZ, false, PACKED>(st, BW, cbase, fu, U, U2, cZ, Hm1, aZ, acc);
+                        direct_update<TZ, false, PACKED>(sbase, row_bytes, fu, U, U2, cZ, Hm1, aZ, acc);
                 } else {
                     atomicOr(P.err, ERR_BOX_OVERFLOW);
                 }
