@@ -31,6 +31,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 #include <cudaTypedefs.h>
 
@@ -969,8 +970,8 @@ __global__ void __launch_bounds__(TX *TY, 2)
 }
 
 // ---------------------------------------------------------------------------
-// Forward projector with slice lanes (the default form; same weights, masks,
-// box and drain as fp_scatter_kernel).  Lane l of warp w holds slice z0 + l
+// Forward projector with slice lanes (where fp_rows_kernel does not apply; same
+// weights, masks, box and drain as fp_scatter_kernel).  Lane l of warp w holds slice z0 + l
 // of the warp's 32 voxel columns (tile rows 2w and 2w+1), and the warp walks
 // its columns one by one.  The lanes of one shared atomic then sit on the
 // rows of 32 consecutive slices of one column: distinct rows whenever the
@@ -993,16 +994,7 @@ __global__ void __launch_bounds__(TX *TY, 2)
 // resolution is 2^-(hb + kb) of the tile's largest contribution (2^-34 or
 // finer) against FP32 atomics' rounding of every partial sum.  The drain
 // forms (hi + lo 2^-kb) / s in FP32.  For finite inputs.
-// FIXED 2 (cbits <= 9) drops the hi word's bias subtraction: the bits of
-// c + 1.5 2^23 are 0x4B400000 + round(c), and 0x4B400000 is a multiple of
-// 2^22, so the low 22 bits of a cell's sum of raw bits are its sum of round(c)
-// modulo 2^22, exact while that sum stays inside +-2^21 (hb = 20 - cbits); the
-// drain sign-extends them.  The lo word keeps its subtraction, with
-// kb = min(22, 30 - cbits): resolution 2^-(hb + kb), 2^-32 or finer.
-// FIXED 3 (cbits <= 8) windows the lo word the same way (kb = 21 - cbits, its
-// cell sums also inside +-2^20): no subtraction at all, resolution 2^-25 or
-// finer.  FIXED 1 takes both subtractions (any cbits <= 13); 0 the FP32 atomics.
-template <int TX, int TY, bool PARTIAL, int FIXED = 0>
+template <int TX, int TY, bool PARTIAL, bool FIXED>
 __global__ void __launch_bounds__(TX *TY, 2)
     fp_scatter_col_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ BPParams P,
                           const float *__restrict__ vin, float u2max, int cbits)
@@ -1071,8 +1063,7 @@ __global__ void __launch_bounds__(TX *TY, 2)
 #pragma unroll
         for (int k = 0; k < NW; ++k) m = fmaxf(m, s_gmax[k]);
         const float cmax = m * u2max;
-        const int hb = FIXED >= 2 ? 20 - cbits : min(30 - cbits, 22);
-        const int kb = FIXED == 3 ? 21 - cbits : FIXED == 2 ? min(22, 30 - cbits) : hb;
+        const int hb = min(30 - cbits, 22), kb = hb;
         int e = 0;
         if (cmax > 0.f && cmax <= 3.0e38f) {
             int ex;
@@ -1132,14 +1123,8 @@ __global__ void __launch_bounds__(TX *TY, 2)
                             const float hm = __fadd_rn(c, kMagic);
                             const float r = __fsub_rn(c, __fsub_rn(hm, kMagic));
                             const float lm = __fmaf_rn(r, lo_scale, kMagic);
-                            if constexpr (FIXED >= 2)
-                                atomicAdd(reinterpret_cast<unsigned *>(acc_hi) + k, __float_as_uint(hm));
-                            else
-                                atomicAdd(acc_hi + k, __float_as_int(hm) - kMagicBits);
-                            if constexpr (FIXED == 3)
-                                atomicAdd(reinterpret_cast<unsigned *>(acc_lo) + k, __float_as_uint(lm));
-                            else
-                                atomicAdd(acc_lo + k, __float_as_int(lm) - kMagicBits);
+                            atomicAdd(acc_hi + k, __float_as_int(hm) - kMagicBits);
+                            atomicAdd(acc_lo + k, __float_as_int(lm) - kMagicBits);
                         };
                         put(o, w0 - w0 * fv);
                         put(o + 1, w1 - w1 * fv);
@@ -1162,9 +1147,7 @@ __global__ void __launch_bounds__(TX *TY, 2)
             const int r = i / BW, c = i - r * BW;
             const int k = r * BWp + c;
             if constexpr (FIXED) {
-                const int hs = FIXED >= 2 ? (int)((unsigned)acc_hi[k] << 10) >> 10 : acc_hi[k];
-                const int ls = FIXED == 3 ? (int)((unsigned)acc_lo[k] << 10) >> 10 : acc_lo[k];
-                st[i] = fmaf((float)ls, lo_unit, (float)hs) * fx_inv;
+                st[i] = fmaf((float)acc_lo[k], lo_unit, (float)acc_hi[k]) * fx_inv;
                 acc_hi[k] = 0;
                 acc_lo[k] = 0;
             } else {
@@ -1180,6 +1163,362 @@ __global__ void __launch_bounds__(TX *TY, 2)
         }
     }
     if (tid == 0) bulk_wait_group_all();
+}
+
+// ---------------------------------------------------------------------------
+// Forward projector with row lanes (the default form).
+//
+// The transpose of the column walk splits into two one-dimensional steps: for
+// one voxel column and projection, the column's slices add to detector rows
+// with the hat weights of v, and the row sums add to detector columns c, c + 1
+// with (1 - fu), fu.  Here a lane owns two detector rows of the box, r and
+// r + 32, and gathers: for each it reads the K slices with |v_z - r| < 1
+// (K = 2 where the row step |scale| U is at least one, 3 from 2/3, 4 from 1/2)
+// from the tile's voxels in shared memory and adds the row sum to registers
+// that stand for the even and the odd one of columns c, c + 1.  A register
+// goes to the box only when its column changes; the columns are walked in the
+// direction in which u changes slower, so that happens about every other
+// column.  No other lane touches the row: the box needs no atomics, and its
+// sums are FP32.
+//
+// A CTA holds 16 x 8 columns of TZ slices; the host picks TZ so that a box has
+// at most 64 rows, the two per lane (rows a column does not reach are computed
+// for nothing: 64 / TZ rows per slice).  Each of the eight warps takes its own
+// projections into its own box and adds it to the gradient by one TMA reduce,
+// so no warp waits for another.  Per projection a warp (1) forms the 128
+// columns' geometry, four per lane, and the box origin, the smallest row and
+// column reached; (2) clears its box and tabulates half of the columns at a
+// time; (3) walks them; (4) hands the box to the TMA.
+//
+// v_z is formed with the roundings of slice_v on the slice table of
+// bp_tma_kernel (z + zoff, times scale, one FMA), so masks and weights are that
+// kernel's voxel by voxel; a slice estimate that rounds to a neighbour loses
+// only weights of a few ulps, because the hat is continuous.
+//
+// Bound by issue (66 %, 56 warp-instructions per 32 updates) beside the shared
+// pipe (58 %).  The scatter with slice lanes and two-word integer atomics
+// (fp_scatter_col_kernel) took 62 instructions and 16.7 shared wavefronts, eight
+// atomics of two wavefronts each, for the same (here 12.2).  Measured, that form
+// -> this one: 512^3 at scale 1.5 into 360 x 768^2 94.9 -> 73.8 ms; 256^2 x 224
+// at scale 1.2 into 240 x 320 x 272 7.71 -> 5.56 ms; 256^3 at scale 1 into
+// 180 x 256^2 5.63 -> 4.08 ms; 48^2 x 40 into 60 x 64^2 0.331 -> 0.133 ms.
+struct FpRows {
+    int TZ;       // slices of a chunk
+    int GP;       // voxels of a column in shared memory, padding included (odd)
+    int nsplit;   // CTAs that share a tile's projections
+};
+
+constexpr int kFpTX = 16, kFpTY = 8, kFpCols = kFpTX * kFpTY, kFpHalf = kFpCols / 2, kFpWarps = 8, kFpMaxRows = 64;
+
+// Packed FP32 pairs.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2_rm(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+template <int K>
+__global__ void __launch_bounds__(32 * kFpWarps, 2)
+    fp_rows_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ BPParams P,
+                   const float *__restrict__ vin, const FpRows R)
+{
+    // padding below the first slice: the smallest slice index a clamped estimate gives is -kPad
+    constexpr int kPad = K == 2 ? 1 : K;
+    constexpr int NT = 32 * kFpWarps;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int BW = P.BW, BH = P.BH, TZ = R.TZ;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    // per warp a box of 64 rows of BW cells (the reduce takes the first BH), per warp a table of half the
+    // columns, the voxels [column][GP]
+    float *box = reinterpret_cast<float *>(smem) + (size_t)w * P.stage_elems;
+    float4 *tabs = reinterpret_cast<float4 *>(reinterpret_cast<float *>(smem) + kFpWarps * (size_t)P.stage_elems);
+    float4 *tab = tabs + w * 2 * kFpHalf;
+    float *vox = reinterpret_cast<float *>(tabs + kFpWarps * 2 * kFpHalf);
+
+    const int2 tile = make_int2((int)(blockIdx.x % (unsigned)P.tilesX), (int)(blockIdx.x / (unsigned)P.tilesX));
+    const int x0 = tile.x * kFpTX, y0 = tile.y * kFpTY;
+    const int z0 = blockIdx.y * TZ, zlast = min(TZ, P.nz - z0) - 1;
+    auto in_fov = [&](int x, int y) {
+        const float aX = flip(P.scale * ((float)x + P.dX), P.dirx);
+        const float aY = flip(P.scale * ((float)y + P.dY), P.diry);
+        return x < P.X && y < P.Y && sqrtf(aX * aX + aY * aY) < P.halfW;
+    };
+    if (!__syncthreads_or(tid < kFpCols && in_fov(x0 + (tid & 15), y0 + (tid >> 4)))) return;  // nothing projects
+
+    // v grows with the slice index sg z: voxels are kept in that order
+    const float ss = flip(P.scale, P.dirz);
+    const bool up = ss > 0.f;
+    for (int i = tid; i < kFpCols * R.GP; i += NT) vox[i] = 0.f;
+    __syncthreads();
+    for (int i = tid; i < kFpCols * (zlast + 1); i += NT) {
+        const int c = i % kFpCols, z = i / kFpCols;
+        const int x = x0 + (c & 15), y = y0 + (c >> 4);
+        if (in_fov(x, y))
+            vox[c * R.GP + kPad + (up ? z : TZ - 1 - z)] =
+                P.fscale * vin[(size_t)(z0 + z) * P.slice_stride + (size_t)y * P.X + x];
+    }
+    __syncthreads();
+
+    const float sg = up ? 1.f : -1.f;
+    const int zf = up ? z0 : z0 + TZ - 1;  // the first slice in walking order
+    const float kz = up ? (float)(zf - kPad) - kMagic : (float)(zf + kPad) + kMagic;
+    const float aZw = flip(P.scale * ((float)zf + P.zoff), P.dirz);
+    const float aZf = flip(P.scale * ((float)z0 + P.zoff), P.dirz);
+    const float aZl = flip(P.scale * ((float)(z0 + zlast) + P.zoff), P.dirz);
+    const float cZ = P.cZ, Hm1 = P.Hm1;
+    const float span = (float)(K == 2 ? TZ + 1 : TZ + K), inv_span = 1.f / span;  // clamp range of the estimate
+    const f32x2 sg2 = pack2(sg, sg), kz2 = pack2(kz, kz), zoff2 = pack2(P.zoff, P.zoff), ss2 = pack2(ss, ss),
+                cZ2 = pack2(cZ, cZ), span2 = pack2(span, span), magic2 = pack2(kMagic, kMagic);
+    const uint32_t vox_s = smem_u32(vox) - 4u * (uint32_t)kMagicBits;
+    // this lane's rows: lane and lane + 32; a row's cell c sits at c ^ sw, sw = (row / 8) mod 4, so that the 32
+    // rows of an access hit 32 banks (BW / 4 is odd) although rows start 16-byte aligned for the TMA
+    const int ra = lane, rb = lane + 32;
+    const uint32_t sw = (uint32_t)(lane >> 3) & 3u;
+    float *rowa = box + (size_t)ra * BW, *rowb = box + (size_t)rb * BW;
+    const uint32_t rowa_s = smem_u32(rowa), row_gap = 32u * 4u * (uint32_t)BW;
+    const float rho_a = (float)ra, rho_b = (float)rb;
+    const int step = kFpWarps * R.nsplit;
+
+    for (int b = (int)blockIdx.z * kFpWarps + w; b < P.N; b += step) {
+        // (1) the geometry of columns lane + 32 k, in the walking order of this projection
+        const float2 cs = P.trig[b];
+        const bool along_x = fabsf(cs.y) <= fabsf(cs.x);  // |du/dx| = |sin|, |du/dy| = |cos| (times scale U)
+        float U[4], u[4];
+        int cu[4], rl[4], rh[4];
+        bool on[4], masked = false;
+        int mc = 0x7fffffff, mr = 0x7fffffff;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int j = lane + 32 * k;
+            const int x = x0 + (along_x ? j & 15 : j >> 3), y = y0 + (along_x ? j >> 4 : j & 7);
+            U[k] = 1.f;
+            u[k] = 0.f;
+            float vlo = 0.f, vhi = 0.f;
+            on[k] = in_fov(x, y);
+            if (on[k]) {
+                const float aX = flip(P.scale * ((float)x + P.dX), P.dirx);
+                const float aY = flip(P.scale * ((float)y + P.dY), P.diry);
+                column_geometry(aX, aY, cs, P.D, P.cX, U[k], u[k]);
+                const float v0 = slice_v(aZf, U[k], cZ), vL = slice_v(aZl, U[k], cZ);
+                vlo = fmaxf(fminf(v0, vL), 0.f);
+                vhi = fminf(fmaxf(v0, vL), Hm1);
+                on[k] = u[k] >= 0.f && u[k] <= P.Wm1 && vlo <= vhi;
+                masked |= on[k] && (fminf(v0, vL) < 0.f || fmaxf(v0, vL) > Hm1);
+            }
+            cu[k] = __float_as_int(__fadd_rd(u[k], kMagic)) - kMagicBits;
+            rl[k] = (int)floorf(vlo);
+            rh[k] = (int)floorf(vhi) + 1;
+            if (on[k]) {
+                mc = min(mc, cu[k]);
+                mr = min(mr, rl[k]);
+            }
+        }
+        const int bx0 = __reduce_min_sync(0xffffffffu, mc) & ~3;  // a TMA coordinate: 16 bytes
+        const int by0 = __reduce_min_sync(0xffffffffu, mr);
+        if (by0 == 0x7fffffff) continue;  // no column reaches the detector
+        const bool any_masked = __any_sync(0xffffffffu, masked);
+        if (lane == 0) bulk_wait_group_read<0>();  // the warp's last reduce has read the box
+        __syncwarp();
+
+        // (2) clear this lane's rows
+        for (int c = 0; c < BW; c += 4) {
+            *reinterpret_cast<float4 *>(rowa + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<float4 *>(rowb + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        // the table entry of column j: (U, A, B, voxel address), then its weights for the even and the odd one of
+        // the detector columns c, c + 1 (U^2 (1 - fu) for c, U^2 fu for c + 1) and their byte offsets in a row.
+        // The columns reached are stored one after another from slot n on.
+        int n = 0;
+        auto entry = [&](int k) {
+            const int j = lane + 32 * k;
+            const int c = cu[k] - bx0;
+            const bool fits = c + 1 < BW && rh[k] - by0 < BH;
+            if (on[k] && !fits) atomicOr(P.err, ERR_BOX_OVERFLOW);
+            const unsigned here = __ballot_sync(0xffffffffu, on[k] && fits);
+            if (on[k] && fits) {
+                // slice estimate (in walking order, kPad at slice 0) of box row rho: span sat(A rho + B)
+                const float A = __frcp_rn(fabsf(ss) * U[k]);
+                const float vw = slice_v(aZw, U[k], cZ);
+                const float pos = fmaf((float)by0 - vw, A, K == 2 ? 1.f : (float)(K + 1) - A);
+                const float fu = u[k] - (float)cu[k];
+                const float U2 = __fmul_rn(U[k], U[k]);
+                const float w1 = U2 * fu, w0 = U2 - w1;
+                const int col = along_x ? j : (j >> 3) + (j & 7) * kFpTX;
+                const bool odd = c & 1;
+                float4 *e = tab + 2 * (n + __popc(here & ((1u << lane) - 1u)));
+                e[0] = make_float4(U[k], A * inv_span, pos * inv_span, __uint_as_float(vox_s + 4u * (uint32_t)(col * R.GP)));
+                e[1] = make_float4(odd ? w1 : w0, odd ? w0 : w1, __int_as_float(4 * (odd ? c + 1 : c)),
+                                   __int_as_float(4 * (odd ? c : c + 1)));
+            }
+            n += __popc(here);
+        };
+
+        // (3) the walk
+        const float rfa = (float)(by0 + ra), rfb = (float)(by0 + rb);
+        // sums of the two rows over the columns whose even cell is pe, odd cell po (byte offsets)
+        float ea = 0.f, eb = 0.f, oa = 0.f, ob = 0.f;
+        uint32_t pe = 0u, po = 4u;
+        auto put = [&](uint32_t cell, float va, float vb) {
+            const uint32_t aa = rowa_s + (cell ^ (4u * sw)), ab = aa + row_gap;
+            float qa, qb;
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(qa) : "r"(aa));
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(qb) : "r"(ab));
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(aa), "f"(qa + va) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(ab), "f"(qb + vb) : "memory");
+        };
+        auto walk = [&](auto mask_tag) {
+            constexpr bool MASK = decltype(mask_tag)::value;
+            auto row_sums = [&](const float4 &e, float &ha, float &hb) {  // per row, the sum over the slices of hat(v - r) g
+                const f32x2 fl = fma2_rm(pack2(__saturatef(fmaf(rho_a, e.y, e.z)), __saturatef(fmaf(rho_b, e.y, e.z))),
+                                         span2, magic2);
+                float fla, flb;
+                unpack2(fl, fla, flb);
+                const uint32_t aa = __float_as_uint(fla) * 4u + __float_as_uint(e.w);
+                const uint32_t ab = __float_as_uint(flb) * 4u + __float_as_uint(e.w);
+                float ga[4], gb[4];
+                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(ga[0]) : "r"(aa));
+                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(gb[0]) : "r"(ab));
+                asm volatile("ld.shared.f32 %0, [%1+4];" : "=f"(ga[1]) : "r"(aa));
+                asm volatile("ld.shared.f32 %0, [%1+4];" : "=f"(gb[1]) : "r"(ab));
+                if constexpr (K >= 3) {
+                    asm volatile("ld.shared.f32 %0, [%1+8];" : "=f"(ga[2]) : "r"(aa));
+                    asm volatile("ld.shared.f32 %0, [%1+8];" : "=f"(gb[2]) : "r"(ab));
+                }
+                if constexpr (K >= 4) {
+                    asm volatile("ld.shared.f32 %0, [%1+12];" : "=f"(ga[3]) : "r"(aa));
+                    asm volatile("ld.shared.f32 %0, [%1+12];" : "=f"(gb[3]) : "r"(ab));
+                }
+                const f32x2 U2v = pack2(e.x, e.x);
+                f32x2 z = fma2(fl, sg2, kz2);  // the slice index (exact)
+                f32x2 s = 0;
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    if (k > 0) z = add2(z, sg2);
+                    float va, vb;
+                    // slice_v(scale * (z + zoff), U, cZ) with its roundings
+                    unpack2(fma2(mul2(add2(z, zoff2), ss2), U2v, cZ2), va, vb);
+                    float wa, wb;
+                    if constexpr (K > 2) {
+                        wa = __saturatef(1.f - fabsf(va - rfa));
+                        wb = __saturatef(1.f - fabsf(vb - rfb));
+                    } else if (k == 0) {  // v <= r
+                        wa = __saturatef(va + (1.f - rfa));
+                        wb = __saturatef(vb + (1.f - rfb));
+                    } else {  // v > r
+                        wa = __saturatef((1.f + rfa) - va);
+                        wb = __saturatef((1.f + rfb) - vb);
+                    }
+                    if (MASK) {  // kernel.cu:130-131
+                        wa = (va >= 0.f && va <= Hm1) ? wa : 0.f;
+                        wb = (vb >= 0.f && vb <= Hm1) ? wb : 0.f;
+                    }
+                    s = k == 0 ? mul2(pack2(wa, wb), pack2(ga[k], gb[k])) : fma2(pack2(wa, wb), pack2(ga[k], gb[k]), s);
+                }
+                unpack2(s, ha, hb);
+            };
+            auto add = [&](float ha, float hb, const float4 &e) {
+                const uint32_t ce = __float_as_uint(e.z), co = __float_as_uint(e.w);
+                if (ce != pe) {  // the same for the whole warp
+                    put(pe, ea, eb);
+                    ea = eb = 0.f;
+                    pe = ce;
+                }
+                if (co != po) {
+                    put(po, oa, ob);
+                    oa = ob = 0.f;
+                    po = co;
+                }
+                ea = fmaf(ha, e.x, ea);
+                eb = fmaf(hb, e.x, eb);
+                oa = fmaf(ha, e.y, oa);
+                ob = fmaf(hb, e.y, ob);
+            };
+            int j = 0;
+            for (; j + 1 < n; j += 2) {
+                const float4 g0 = tab[2 * j], g1 = tab[2 * j + 2];
+                float h0a, h0b, h1a, h1b;
+                row_sums(g0, h0a, h0b);
+                row_sums(g1, h1a, h1b);
+                add(h0a, h0b, tab[2 * j + 1]);
+                add(h1a, h1b, tab[2 * j + 3]);
+            }
+            if (j < n) {
+                float ha, hb;
+                row_sums(tab[2 * j], ha, hb);
+                add(ha, hb, tab[2 * j + 1]);
+            }
+        };
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+            __syncwarp();  // the walk over the first half is done with the table
+            n = 0;
+            if (h == 0) {
+                entry(0);
+                entry(1);
+            } else {
+                entry(2);
+                entry(3);
+            }
+            __syncwarp();
+            if (any_masked)
+                walk(std::true_type{});
+            else
+                walk(std::false_type{});
+        }
+        put(pe, ea, eb);
+        put(po, oa, ob);
+
+        // (4) undo the rows' column order in place, then reduce the box into the gradient
+        auto unswizzle = [&](float *row) {
+            for (int c = 0; c < BW; c += 4) {
+                float4 q = *reinterpret_cast<float4 *>(row + c);
+                if (sw & 1u) q = make_float4(q.y, q.x, q.w, q.z);
+                if (sw & 2u) q = make_float4(q.z, q.w, q.x, q.y);
+                *reinterpret_cast<float4 *>(row + c) = q;
+            }
+        };
+        if (sw) {
+            unswizzle(rowa);
+            if (rb < BH) unswizzle(rowb);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            tma_reduce_add_3d(&tmap, bx0, by0, b, box);
+            bulk_commit_group();
+        }
+    }
+    if (lane == 0) bulk_wait_group_all();
 }
 
 // ---------------------------------------------------------------------------
@@ -1295,8 +1634,7 @@ static const BPVariant kVariants[] = {
 
 static int g_variant_override = -1;  // index into kVariants, set by tk_bp_select_variant
 static int g_diag_box_shrink = 0;    // rows taken off every staged box (tk_diag_shrink_box)
-static int g_fp_variant = 0;  // forward projector: 0 slice lanes, fixed-point box; 1 column lanes; 2 slice lanes,
-                              // FP32 atomics
+static int g_fp_variant = 0;  // forward projector: 0 row lanes; 1 column lanes; 2 slice lanes, FP32 atomics
 
 static const BPVariant *pick_variant(int precision)
 {
@@ -1558,6 +1896,51 @@ int launch_backproject_quarter(const tk_geometry &g, const void *d_q, int precis
                           compact);
 }
 
+// Shape of a row-lane forward projection (fp_rows_kernel), or K = 0 where it does not apply: the source
+// inside the field of view (U has no bound there), row steps below 1/2 (more than four slices per row), or
+// footprints too large for two CTAs per SM.
+struct FpRowsPlan {
+    int K = 0, TZ = 0, GP = 0, zchunks = 0, BW = 0, BH = 0, stage_elems = 0;
+    size_t smem = 0;
+};
+
+// The box of a 16 x 8 x TZ tile measured from the smallest row and column that its columns inside the field of
+// view reach: columns 0 .. floor(du) + 1 (plus the second tap, plus 3 for the TMA alignment of the origin),
+// rows 0 .. floor(dv) + 2, with du, dv bounded as in bp_box_dims for radii up to W/2.
+static FpRowsPlan fp_rows_plan(const tk_geometry &g, int nz, float zoff)
+{
+    FpRowsPlan p;
+    const double s = std::fabs((double)g.scale), D = g.D;
+    const double ex = s * std::fmax(std::fabs((double)g.cx), std::fabs((double)(g.X - 1) - g.cx));
+    const double ey = s * std::fmax(std::fabs((double)g.cy), std::fabs((double)(g.Y - 1) - g.cy));
+    const double R = std::fmin(0.5 * g.W, std::sqrt(ex * ex + ey * ey) + 1.0);
+    if (!(D - R > 1e-3 * D)) return p;
+    const double dv_min = s * D / (D + R);
+    const int K = dv_min >= 1.0001 ? 2 : dv_min >= 2.0001 / 3.0 ? 3 : dv_min >= 0.50005 ? 4 : 0;
+    if (!K) return p;
+    const double Umax = D / (D - R), dU = D / ((D - R) * (D - R));
+    const double dxy = s * std::sqrt((double)((kFpTX - 1) * (kFpTX - 1) + (kFpTY - 1) * (kFpTY - 1)));
+    const double azmax = s * std::fmax(std::fabs((double)zoff), std::fabs((double)(nz - 1) + zoff));
+    const int BW = (((int)std::floor(dxy * Umax + R * dU * dxy + 0.01) + 6 + 3) / 4 | 1) * 4;  // BW / 4 odd
+    if (BW > 256) return p;
+    auto shape = [&](int TZ) {
+        p.TZ = TZ;
+        p.GP = (TZ + (K == 2 ? 3 : 2 * K)) | 1;
+        p.BW = BW;
+        p.BH = (int)std::floor(s * (TZ - 1) * Umax + azmax * dU * dxy + 0.01) + 3;
+        p.stage_elems = BW * kFpMaxRows;
+        p.smem = kFpWarps * ((size_t)p.stage_elems * 4 + 2 * kFpHalf * sizeof(float4)) + (size_t)kFpCols * p.GP * 4;
+        return p.BH <= kFpMaxRows && p.smem <= 112 * 1024;  // two CTAs per SM
+    };
+    int TZ = std::min(nz, kFpMaxRows);
+    while (TZ >= 1 && !shape(TZ)) --TZ;
+    if (TZ < std::min(nz, 8)) return p;
+    p.zchunks = (nz + TZ - 1) / TZ;
+    shape((nz + p.zchunks - 1) / p.zchunks);  // even chunks
+    p.K = K;
+    return p;
+}
+
 int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, float zoff, float *d_qbar,
                            int accumulate, cudaStream_t stream)
 {
@@ -1575,16 +1958,23 @@ int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, flo
     const BPVariant shape = {nullptr, nullptr, TK_F32, TX, TY, TZ, 2, false, "fp"};
     int BW, BH;
     if (int rc = bp_box_dims(g, nz, zoff, shape.TX, shape.TY, shape.TZ, shape.coef, 4, &BW, &BH)) return rc;
+    FpRowsPlan rows;
+    if (g_fp_variant == 0) rows = fp_rows_plan(g, nz, zoff);
+    const int boxBW = BW, boxBH = BH;  // of the slice-lane and column-lane forms
+    if (rows.K) {
+        BW = rows.BW;
+        BH = rows.BH;
+    }
     std::vector<float> cs(g.N), sn(g.N);
     build_trig(g, cs.data(), sn.data());
     const int p = reference_pad_length(g.W);
-    const int tilesX = (g.X + TX - 1) / TX, tilesY = (g.Y + TY - 1) / TY;
-    const int zchunks = (nz + TZ - 1) / TZ;
+    const int tilesX = (g.X + TX - 1) / TX, tilesY = rows.K ? (g.Y + kFpTY - 1) / kFpTY : (g.Y + TY - 1) / TY;
+    const int zchunks = rows.K ? rows.zchunks : (nz + TZ - 1) / TZ;
     TK_CHECK((long long)tilesX * tilesY < (1ll << 31) && zchunks < 65536, TK_ERR_UNSUPPORTED,
              "volume too large for one launch");
     const bool partial = nz < TZ;
-    // Slice lanes with the two-word fixed-point box (variant 0, the default), column lanes (1), or
-    // slice lanes with FP32 shared atomics (2).  The fixed-point box needs a bound on the contributions that
+    // Row lanes (variant 0, the default) or, where fp_rows_plan finds no shape, slice lanes with the two-word
+    // fixed-point box; column lanes (1); slice lanes with FP32 shared atomics (2).  The fixed-point box needs a bound on the contributions that
     // reach one cell of one projection from one tile (a cell takes the voxels whose u lies in a
     // 2-pixel band and whose v lies in a 2-row band):
     //  - the columns whose u falls in a 2-pixel band lie between two rays from the source, a strip
@@ -1611,18 +2001,12 @@ int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, flo
     if (!cols)
         fn = partial ? reinterpret_cast<const void *>(&fp_scatter_kernel<TX, TY, true>)
                      : reinterpret_cast<const void *>(&fp_scatter_kernel<TX, TY, false>);
-    else if (fixed && cbits <= 8)
-        fn = partial ? reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, true, 3>)
-                     : reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, false, 3>);
-    else if (fixed && cbits <= 9)
-        fn = partial ? reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, true, 2>)
-                     : reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, false, 2>);
     else if (fixed)
-        fn = partial ? reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, true, 1>)
-                     : reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, false, 1>);
+        fn = partial ? reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, true, true>)
+                     : reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, false, true>);
     else
-        fn = partial ? reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, true, 0>)
-                     : reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, false, 0>);
+        fn = partial ? reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, true, false>)
+                     : reinterpret_cast<const void *>(&fp_scatter_col_kernel<TX, TY, false, false>);
 
     static thread_local BPParams P;
     std::memset(&P, 0, sizeof(P));
@@ -1634,7 +2018,7 @@ int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, flo
     P.nz = nz;
     P.BW = BW;
     P.BH = BH;
-    P.stage_elems = (BW * BH + 31) / 32 * 32;  // 128-byte aligned boxes
+    P.stage_elems = rows.K ? rows.stage_elems : (BW * BH + 31) / 32 * 32;  // 128-byte aligned boxes
     P.tilesX = tilesX;
     P.tilesY = tilesY;
     P.cX = g.cX;
@@ -1667,14 +2051,33 @@ int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, flo
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         TK_CHECK(cr == CUDA_SUCCESS, TK_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)cr);
         // odd-pitch accumulation box (two words per cell in the fixed-point form)
-        const size_t acc_elems = (size_t)((BH * (BW + 1) + 31) & ~31) * (fixed ? 2 : 1);
+        const size_t acc_elems = (size_t)((boxBH * (boxBW + 1) + 31) & ~31) * (fixed ? 2 : 1);
         const size_t geo_bytes = cols ? (size_t)(TX * TY / 32) * 32 * sizeof(float4) : 0;  // slice-lane form
-        const size_t smem = (2 * (size_t)P.stage_elems + acc_elems) * sizeof(float) + geo_bytes +
+        const size_t smem = (2 * (size_t)((boxBW * boxBH + 31) / 32 * 32) + acc_elems) * sizeof(float) + geo_bytes +
                             (size_t)nb * sizeof(int2) + 16;
         TK_CHECK(smem <= 227 * 1024, TK_ERR_UNSUPPORTED, "forward project: %zu B of shared memory needed", smem);
+        const float *vin = d_vol;
+        if (rows.K) {
+            const void *rfn = rows.K == 2   ? reinterpret_cast<const void *>(&fp_rows_kernel<2>)
+                              : rows.K == 3 ? reinterpret_cast<const void *>(&fp_rows_kernel<3>)
+                                            : reinterpret_cast<const void *>(&fp_rows_kernel<4>);
+            int dev = 0, sms = 0;
+            TK_CUDA(cudaGetDevice(&dev));
+            TK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            // small volumes: several CTAs per tile, each its share of the projections (at least 4 per warp),
+            // until the chip has about four waves of CTAs
+            const long long ctas = (long long)tilesX * tilesY * zchunks;
+            const int split = (int)std::max(1ll, std::min<long long>((8ll * sms + ctas - 1) / ctas, nb / (4 * kFpWarps)));
+            FpRows fr{rows.TZ, rows.GP, split};
+            TK_CUDA(cudaFuncSetAttribute(rfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows.smem));
+            void *args_fr[] = {&tmap, &P, &vin, &fr};
+            TK_CUDA(cudaLaunchKernel(rfn, dim3((unsigned)(tilesX * tilesY), (unsigned)zchunks, (unsigned)split),
+                                     dim3(32 * kFpWarps), args_fr, rows.smem, stream));
+            count_launch();
+            continue;
+        }
         TK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         dim3 grid((unsigned)(tilesX * tilesY), partial ? 1u : (unsigned)zchunks, 1);
-        const float *vin = d_vol;
         float u2 = u2max;
         int cb = cbits;
         void *args_cols[] = {&tmap, &P, &vin, &u2, &cb};
