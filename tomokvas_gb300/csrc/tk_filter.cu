@@ -10,9 +10,9 @@
 // GB300 design: one pass over HBM.  Each CTA streams pairs of detector rows
 // straight from the raw input, applies log + cosine weight while loading,
 // packs the two real rows as one complex signal z = a + i b, and runs a
-// radix-4/2 Stockham FFT in shared memory.  Because the filter spectrum is
-// real and even, IFFT(FFT(z) * Hf) = (a*k) + i (b*k), so one forward and one
-// inverse complex FFT filter two rows.  The inverse is computed as
+// radix-16 Stockham FFT in registers and shared memory.  Because the filter
+// spectrum is real and even, IFFT(FFT(z) * Hf) = (a*k) + i (b*k), so one forward
+// and one inverse complex FFT filter two rows.  The inverse is computed as
 // conj(FFT(conj(Z) * Hf)).  Results are written once, projection-major, in
 // FP32/FP16/BF16.  No cuFFT, no staging copies, no per-row plans.
 #include "tk_common.cuh"
@@ -33,40 +33,61 @@ constexpr int kFiltThreads = 256;
 constexpr float kScaleTarget = 16384.f;  // bound of |stored value| for 16-bit storage
 
 // ---------------------------------------------------------------------------
-// Mixed-radix Stockham FFT in shared memory.
+// Mixed-radix Stockham FFT.
 //
-// A length p = 2^lg transform runs as radix-16 passes and one final radix
-// 8/4/2 pass (p = 2048: 16, 16, 8).  Pass m with span Ns and radix R maps
-// butterfly j (k = j mod Ns) as
+// A pass with span Ns and radix R maps butterfly j (k = j mod Ns) as
 //   v[r] = x[j + r p/R] * w^(r k p/(R Ns)),  y[(j-k) R + k + s Ns] = DFT_R(v)[s],
-// one butterfly per thread, the R points in registers.  Buffers are padded by
-// one element per 16 (pidx), which makes every pass's loads and stores
-// conflict-free; twiddles come from per-pass tables laid out [k][r] (one
-// thread reads R-1 consecutive entries).
-struct FFTPlan {
-    int npass;
-    int R[5], Ns[5], off[5];  // radix, span and twiddle-table offset of each pass
-    int tw_total;             // twiddle entries of all passes
-};
+// one butterfly per thread, the R points in registers.  The length p = 2^lg
+// forward transform runs radix 16 passes and one last pass of radix
+// RL = 16, 8, 4 or 2; the inverse runs the RL pass first.  Then three of the
+// joints need no shared memory: the first forward pass (Ns = 1) takes the
+// samples x[j + r p/16] from registers, its upper half being the zero padding;
+// the last forward pass ends on X[j + s p/RL], which are just the inputs of the
+// inverse's first pass, so spectrum product and both butterflies run on the
+// same registers; and the last inverse pass (Ns = p/16) ends on the output
+// columns j + s p/16, of which s < 8 are wanted.  A row pair of p = 2048 takes
+// four passes through shared memory and five barriers (eight and nine with a
+// separate load, product and output pass): 90 frames of 1024^2 uint16 into FP16
+// coefficients 830 -> 668 us, 411 x 300 FP32 rows of 1501 (p = 4096)
+// 1971 -> 1310 us.
+//
+// Buffers are padded by one element per 16 (pidx), which makes every pass's
+// loads and stores conflict-free; twiddles come from per-pass tables laid out
+// [k][r] (one thread reads R-1 consecutive entries).
 
-__host__ __device__ inline FFTPlan fft_plan(int lg)
+// Threads per transform (one radix-16 butterfly each); compile-time form.
+__host__ __device__ constexpr int fft_threads_c(int p)
 {
-    FFTPlan pl{};
-    int Ns = 1, rem = lg, off = 0;
-    while (rem > 0) {
-        const int b = rem >= 4 ? 4 : rem;
-        const int R = 1 << b;
-        pl.R[pl.npass] = R;
-        pl.Ns[pl.npass] = Ns;
-        pl.off[pl.npass] = off;
-        if (Ns > 1) off += Ns * (R - 1);
-        Ns *= R;
-        rem -= b;
-        ++pl.npass;
-    }
-    pl.tw_total = off;
-    return pl;
+    return ((p >> 4) > 32 ? (p >> 4) : 32) < kFiltThreads ? ((p >> 4) > 32 ? (p >> 4) : 32) : kFiltThreads;
 }
+
+// Shape of the length-2^LG filter.
+template <int LG> struct Fft {
+    static constexpr int P = 1 << LG, NP = (LG + 3) / 4;              // passes of one transform
+    static constexpr int RL = LG % 4 ? 1 << (LG % 4) : 16;            // radix of the last forward pass
+    static constexpr int R1 = NP > 1 ? 16 : RL, Q1 = P / R1;          // first pass: radix and butterflies
+    static constexpr int TPF = fft_threads_c(P), G = kFiltThreads / TPF;
+    static constexpr int IN = R1 / 2, ITIN = (Q1 + TPF - 1) / TPF;    // samples j + r Q1, r < IN, per butterfly
+    // output columns j + s QC, s < NC, of butterfly j of the last pass
+    static constexpr int NC = NP > 1 ? 8 : 1, QC = NP > 1 ? P / 16 : P / 2, ITC = (QC + TPF - 1) / TPF;
+    // twiddle tables: forward passes m >= 1 (span 16^m), then the inverse's radix-16 passes (span RL 16^m).
+    // RL = 16: the same tables.  LG = 13: the last forward table, w^k for k < p/2, serves the inverse.
+    static constexpr int fwd_off(int m) { return m >= 1 ? (1 << (4 * m)) - 16 : 0; }
+    static constexpr int FWD = NP > 1 ? fwd_off(NP - 1) + (P / RL) * (RL - 1) : 0;
+    static constexpr bool OWN_INV = RL != 16 && LG < 13 && NP > 1;
+    static constexpr int inv_span(int m) { return RL << (4 * m); }    // m = 0 .. NP - 2
+    static constexpr int inv_off(int m)
+    {
+        int o = OWN_INV ? FWD : 0;
+        for (int i = 0; i < m; ++i) o += inv_span(i) * 15;
+        return o;
+    }
+    static constexpr int TW = OWN_INV ? inv_off(NP - 1) : FWD;        // entries of all tables
+    static constexpr int HF = ((P / 2 + 1) + 3) & ~3;                 // spectrum, floats
+    static constexpr int EDGE = (TPF / 32) * (NC + 1);                // first columns of each warp, float2
+    static constexpr size_t group_bytes() { return (size_t)(2 * (P + P / 16) + EDGE) * 8; }
+    static constexpr size_t smem() { return (size_t)TW * 8 + HF * 4 + G * group_bytes(); }
+};
 
 struct FiltParams {
     LoadParams L;
@@ -79,92 +100,54 @@ struct FiltParams {
     int fgrp, fstride;      // coefficient image, frames in groups (> 0): frame f is f/fgrp*fstride + f%fgrp
     int out_layout;         // raw output: TK_LAYOUT_PROJECTION [N][H][Wp] or TK_LAYOUT_SINOGRAM [H][N][Wp]
     int weight_out;         // multiply the output by the cosine weight (the filter's transpose)
-    FFTPlan plan;           // passes of the length-p transform (fft_plan(lg))
     float Hf[kMaxHf];  // tau * |R2C_p(h)| * window, k = 0..p/2
 };
-
-// Raw samples x0 .. x0+NV-1 of the row at element offset off; samples at or
-// past W read as 0.  With L.vec the run is read with 16-byte loads (the run
-// starts on a 16-byte boundary: x0 is a multiple of NV, NV * element size is
-// a multiple of 16, rows start aligned and the row pitch covers every chunk
-// that starts below W).
-template <int NV>
-__device__ __forceinline__ void load_run(const LoadParams &L, long long off, int x0, bool valid, float (&v)[NV])
-{
-#pragma unroll
-    for (int j = 0; j < NV; ++j) v[j] = 0.f;
-    if (!valid) return;
-    if constexpr (NV % 8 == 0) {
-        if (L.vec && L.input_type == TK_INPUT_U16) {
-            const uint4 *src = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(L.in) + off + x0);
-#pragma unroll
-            for (int k = 0; k < NV / 8; ++k) {
-                if (x0 + 8 * k < L.W) {
-                    const uint4 q = __ldg(src + k);
-                    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        v[8 * k + 2 * e] = (float)(w[e] & 0xffffu);
-                        v[8 * k + 2 * e + 1] = (float)(w[e] >> 16);
-                    }
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < NV; ++j)
-                if (x0 + j >= L.W) v[j] = 0.f;
-            return;
-        }
-    }
-    if constexpr (NV % 4 == 0) {
-        if (L.vec && L.input_type == TK_INPUT_F32) {
-            const float4 *src = reinterpret_cast<const float4 *>(static_cast<const float *>(L.in) + off + x0);
-#pragma unroll
-            for (int k = 0; k < NV / 4; ++k) {
-                if (x0 + 4 * k < L.W) {
-                    const float4 q = __ldg(src + k);
-                    v[4 * k] = q.x;
-                    v[4 * k + 1] = q.y;
-                    v[4 * k + 2] = q.z;
-                    v[4 * k + 3] = q.w;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < NV; ++j)
-                if (x0 + j >= L.W) v[j] = 0.f;
-            return;
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NV; ++j)
-        if (x0 + j < L.W) v[j] = load_raw(L, off, x0 + j);
-}
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// Complex sum and difference as one packed FP32 instruction each.
+__device__ __forceinline__ float2 cadd(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 A, B;\n\tmov.b64 A, {%2, %3};\n\tmov.b64 B, {%4, %5};\n\t"
+        "add.rn.f32x2 A, A, B;\n\tmov.b64 {%0, %1}, A;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 csub(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 A, B;\n\tmov.b64 A, {%2, %3};\n\tmov.b64 B, {%4, %5};\n\t"
+        "sub.rn.f32x2 A, A, B;\n\tmov.b64 {%0, %1}, A;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
 
 // Padded index of element i of a transform buffer.
 __host__ __device__ __forceinline__ int pidx(int i) { return i + (i >> 4); }
-__host__ __device__ __forceinline__ int padded_len(int p) { return p + (p >> 4); }
 
-// Twiddle tables of every pass: entry (k, r) of pass m is w^(r k p/(R Ns)) =
-// exp(-2 pi i r k / (R Ns)), r = 1..R-1, k < Ns.  All threads of the CTA.
-__device__ __forceinline__ void fill_twiddles(float2 *twp, const FFTPlan &pl)
+// Twiddle table of a pass: entry (k, r) is exp(-2 pi i r k / (R Ns)), r = 1..R-1, k < Ns.  All threads of the CTA.
+__device__ __forceinline__ void fill_table(float2 *tw, int R, int Ns)
 {
+    for (int i = threadIdx.x; i < Ns * (R - 1); i += blockDim.x) {
+        const int k = i / (R - 1), r = i - k * (R - 1) + 1;
+        float sn, cs;
+        sincospif(-2.0f * (float)(r * k) / (float)(R * Ns), &sn, &cs);  // exact argument: R Ns is 2^n
+        tw[i] = make_float2(cs, sn);
+    }
+}
+template <int LG> __device__ __forceinline__ void fill_twiddles(float2 *tw)
+{
+    using F = Fft<LG>;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        if (m >= pl.npass) break;
-        const int R = pl.R[m], Ns = pl.Ns[m];
-        if (Ns == 1) continue;
-        for (int i = threadIdx.x; i < Ns * (R - 1); i += blockDim.x) {
-            const int k = i / (R - 1), r = i - k * (R - 1) + 1;
-            float sn, cs;
-            sincospif(-2.0f * (float)(r * k) / (float)(R * Ns), &sn, &cs);  // exact argument: R Ns is 2^n
-            twp[pl.off[m] + i] = make_float2(cs, sn);
-        }
+    for (int m = 1; m < F::NP; ++m) fill_table(tw + F::fwd_off(m), m == F::NP - 1 ? F::RL : 16, 1 << (4 * m));
+    if constexpr (F::OWN_INV) {
+#pragma unroll
+        for (int m = 0; m < F::NP - 1; ++m) fill_table(tw + F::inv_off(m), 16, F::inv_span(m));
     }
 }
 
@@ -210,11 +193,17 @@ template <> __device__ __forceinline__ void dft<8>(float2 (&v)[8])
 }
 // 16 = 4 x 4: E_e = DFT4(x[e], x[e+4], x[e+8], x[e+12]); T_e[k] = W16^(e k) E_e[k];
 // X[k + 4h] = DFT4_h(T_0[k], T_1[k], T_2[k], T_3[k]).
-template <> __device__ __forceinline__ void dft<16>(float2 (&v)[16])
+// DFT_4 of (x0, x1, 0, 0).
+__device__ __forceinline__ void dft4_half(float2 x0, float2 x1, float2 &o0, float2 &o1, float2 &o2, float2 &o3)
 {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) dft4(v[e], v[e + 4], v[e + 8], v[e + 12]);
-    // E_e[k] sits in v[e + 4k]; apply W16^(e k)
+    o0 = cadd(x0, x1);
+    o2 = csub(x0, x1);
+    o1 = make_float2(x0.x + x1.y, x0.y - x1.x);
+    o3 = make_float2(x0.x - x1.y, x0.y + x1.x);
+}
+// The W16^(e k) of dft<16> on E_e[k] in v[e + 4k], then its second stage; LOW: outputs 0 .. 7 only.
+template <bool LOW> __device__ __forceinline__ void dft16_second(float2 (&v)[16])
+{
     const float2 w1 = make_float2(kC8, -kS8), w2 = make_float2(kR2, -kR2), w3 = make_float2(kS8, -kC8);
     const float2 w6 = make_float2(-kR2, -kR2), w9 = make_float2(-kC8, kS8);
     v[5] = cmul(v[5], w1);                          // e=1,k=1
@@ -229,68 +218,45 @@ template <> __device__ __forceinline__ void dft<16>(float2 (&v)[16])
     float2 o[16];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        float2 a = v[4 * k], b = v[4 * k + 1], c = v[4 * k + 2], d = v[4 * k + 3];
-        dft4(a, b, c, d);
-        o[k] = a;
-        o[k + 4] = b;
-        o[k + 8] = c;
-        o[k + 12] = d;
+        const float2 x0 = v[4 * k], x1 = v[4 * k + 1], x2 = v[4 * k + 2], x3 = v[4 * k + 3];
+        const float2 a = cadd(x0, x2), b = csub(x0, x2), c = cadd(x1, x3), d = csub(x1, x3);
+        o[k] = cadd(a, c);
+        o[k + 4] = make_float2(b.x + d.y, b.y - d.x);
+        if constexpr (!LOW) {
+            o[k + 8] = csub(a, c);
+            o[k + 12] = make_float2(b.x - d.y, b.y + d.x);
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = o[i];
+    for (int i = 0; i < (LOW ? 8 : 16); ++i) v[i] = o[i];
 }
-
-// Threads per transform (one radix-16 butterfly each); compile-time form.
-__host__ __device__ constexpr int fft_threads_c(int p)
+template <> __device__ __forceinline__ void dft<16>(float2 (&v)[16])
 {
-    return ((p >> 4) > 32 ? (p >> 4) : 32) < kFiltThreads ? ((p >> 4) > 32 ? (p >> 4) : 32) : kFiltThreads;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dft4(v[e], v[e + 4], v[e + 8], v[e + 12]);
+    dft16_second<false>(v);
 }
-
-// Compile-time length: pass m of a length-2^LG transform has radix 16 except
-// possibly the last (fft_plan), span Ns = 16^m and its twiddle table at
-// offset 16^m - 16 (m >= 1).  With every size a constant, the padded
-// addresses of the loads and stores fold into immediates and the butterfly
-// loops unroll.
-template <int R, int P, int NS>
-__device__ __forceinline__ void fft_pass_c(const float2 *__restrict__ x, float2 *__restrict__ y,
-                                           const float2 *__restrict__ tw, int t)
+// Outputs 0 .. 7 of DFT_16.
+__device__ __forceinline__ void dft16_low(float2 (&v)[16])
 {
-    constexpr int Q = P / R;
-    constexpr int TPF = fft_threads_c(P);
-    constexpr int ITER = (Q + TPF - 1) / TPF;
 #pragma unroll
-    for (int i = 0; i < ITER; ++i) {
-        const int j = t + i * TPF;
-        if ((Q % TPF) != 0 && j >= Q) break;
-        const int k = j & (NS - 1);
-        float2 v[R];
-        if constexpr (Q % 16 == 0) {  // pidx(j + r Q) = pidx(j) + r (Q + Q/16)
-            const float2 *xs = x + pidx(j);
+    for (int e = 0; e < 4; ++e) dft4(v[e], v[e + 4], v[e + 8], v[e + 12]);
+    dft16_second<true>(v);
+}
+// DFT_R of R/2 values followed by R/2 zeros.
+template <int R> __device__ __forceinline__ void dft_half(float2 (&v)[R])
+{
+    if constexpr (R == 2) {
+        v[1] = v[0];
+    } else if constexpr (R == 4) {
+        dft4_half(v[0], v[1], v[0], v[1], v[2], v[3]);
+    } else if constexpr (R == 8) {
+        v[4] = v[5] = v[6] = v[7] = make_float2(0.f, 0.f);
+        dft<8>(v);
+    } else {
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = xs[r * (Q + Q / 16)];
-        } else {
-#pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = x[pidx(j + r * Q)];
-        }
-        if constexpr (NS > 1) {
-            const float2 *w = tw + k * (R - 1) - 1;
-#pragma unroll
-            for (int r = 1; r < R; ++r) v[r] = cmul(v[r], w[r]);
-        }
-        dft<R>(v);
-        const int o = (j - k) * R + k;
-        if constexpr (NS % 16 == 0) {
-            float2 *ys = y + pidx(o);
-#pragma unroll
-            for (int s2 = 0; s2 < R; ++s2) ys[s2 * (NS + NS / 16)] = v[s2];
-        } else if constexpr (NS == 1 && R == 16) {  // o is a multiple of 16: o + s stays in one padding group
-            float2 *ys = y + pidx(o);
-#pragma unroll
-            for (int s2 = 0; s2 < R; ++s2) ys[s2] = v[s2];
-        } else {
-#pragma unroll
-            for (int s2 = 0; s2 < R; ++s2) y[pidx(o + s2 * NS)] = v[s2];
-        }
+        for (int e = 0; e < 4; ++e) dft4_half(v[e], v[e + 4], v[e], v[e + 4], v[e + 8], v[e + 12]);
+        dft16_second<false>(v);
     }
 }
 
@@ -302,65 +268,181 @@ __device__ __forceinline__ void group_sync(int grp)
     asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(TPF) : "memory");
 }
 
+// Loads of butterfly j of a radix-R pass: x[j + r Q] times its twiddles.
+template <int R, int P, int NS, bool FROM_HALF>
+__device__ __forceinline__ void load_butterfly(float2 (&v)[R], const float2 *x, const float2 *tw, int j)
+{
+    constexpr int Q = P / R;
+    const int k = j & (NS - 1);
+    if constexpr (Q % 16 == 0) {  // pidx(j + r Q) = pidx(j) + r (Q + Q/16)
+        const float2 *xs = x + pidx(j);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = xs[r * (Q + Q / 16)];
+    } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = x[pidx(j + r * Q)];
+    }
+    if constexpr (NS > 1 && FROM_HALF) {  // tw[m] = w_P^m, m < P/2; w_P^(m + P/2) = -w_P^m
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+            const int m = r * k * (P / (R * NS));
+            float2 w = tw[m & (P / 2 - 1)];
+            if (m & (P / 2)) w = make_float2(-w.x, -w.y);
+            v[r] = cmul(v[r], w);
+        }
+    } else if constexpr (NS > 1) {
+        const float2 *w = tw + k * (R - 1) - 1;
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = cmul(v[r], w[r]);
+    }
+}
+// Its stores: y[(j - k) R + k + s Ns].
+template <int R, int NS> __device__ __forceinline__ void store_butterfly(const float2 (&v)[R], float2 *y, int j)
+{
+    const int k = j & (NS - 1);
+    const int o = (j - k) * R + k;
+    if constexpr (NS % 16 == 0) {
+        float2 *ys = y + pidx(o);
+#pragma unroll
+        for (int s2 = 0; s2 < R; ++s2) ys[s2 * (NS + NS / 16)] = v[s2];
+    } else if constexpr (NS == 1 && R == 16) {  // o is a multiple of 16: o + s stays in one padding group
+        float2 *ys = y + pidx(o);
+#pragma unroll
+        for (int s2 = 0; s2 < R; ++s2) ys[s2] = v[s2];
+    } else {
+#pragma unroll
+        for (int s2 = 0; s2 < R; ++s2) y[pidx(o + s2 * NS)] = v[s2];
+    }
+}
+
+// A radix-16 pass of span NS from x to y and the group's barrier.
+template <int LG, int NS, bool FROM_HALF>
+__device__ __forceinline__ void pass16(const float2 *x, float2 *y, const float2 *tw, int t, int grp)
+{
+    using F = Fft<LG>;
+    constexpr int Q = F::P / 16, ITER = (Q + F::TPF - 1) / F::TPF;
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+        const int j = t + i * F::TPF;
+        if ((Q % F::TPF) != 0 && j >= Q) break;
+        float2 v[16];
+        load_butterfly<16, F::P, NS, FROM_HALF>(v, x, tw, j);
+        dft<16>(v);
+        store_butterfly<16, NS>(v, y, j);
+    }
+    group_sync<F::TPF>(grp);
+}
+// Forward passes m = M .. NP - 2.
 template <int LG, int M>
-__device__ __forceinline__ void fft_passes_c(float2 *&a, float2 *&b, const float2 *twp, int t, int grp)
+__device__ __forceinline__ void forward_passes(float2 *&x, float2 *&y, const float2 *tw, int t, int grp)
 {
-    if constexpr (LG - 4 * M > 0) {
-        constexpr int rem = LG - 4 * M;
-        constexpr int R = rem >= 4 ? 16 : (1 << rem);
-        constexpr int NS = 1 << (4 * M);
-        constexpr int OFF = M >= 1 ? (1 << (4 * M)) - 16 : 0;
-        fft_pass_c<R, (1 << LG), NS>(a, b, twp + OFF, t);
-        group_sync<fft_threads_c(1 << LG)>(grp);
-        float2 *s2 = a;
-        a = b;
-        b = s2;
-        fft_passes_c<LG, M + 1>(a, b, twp, t, grp);
+    using F = Fft<LG>;
+    if constexpr (M <= F::NP - 2) {
+        pass16<LG, (1 << (4 * M)), false>(x, y, tw + F::fwd_off(M), t, grp);
+        float2 *z = x;
+        x = y;
+        y = z;
+        forward_passes<LG, M + 1>(x, y, tw, t, grp);
+    }
+}
+// Inverse radix-16 passes m = M .. NP - 3 (all but the last).
+template <int LG, int M>
+__device__ __forceinline__ void inverse_passes(float2 *&x, float2 *&y, const float2 *tw, int t, int grp)
+{
+    using F = Fft<LG>;
+    if constexpr (M <= F::NP - 3) {
+        if constexpr (LG == 13)
+            pass16<LG, F::inv_span(M), true>(x, y, tw + F::fwd_off(F::NP - 1), t, grp);
+        else
+            pass16<LG, F::inv_span(M), false>(x, y, tw + F::inv_off(M), t, grp);
+        float2 *z = x;
+        x = y;
+        y = z;
+        inverse_passes<LG, M + 1>(x, y, tw, t, grp);
     }
 }
 
-// Forward FFT of length 2^LG (padded buffers); ping-pongs between a and b and
-// returns the buffer holding the result.  Every thread of the transform group
-// calls it (group barriers inside).
+// Filters one row pair.  in[i][r] is the packed sample x = j + r Q1 of butterfly j = t + i TPF (the caller's
+// registers; 0 at x >= W), out[i][s] the filtered pair (a, -b) at column j + s QC of butterfly j = t + i TPF.  Every
+// thread of the group calls it.  Buffer A is free again when it returns, B once the group has passed another barrier.
 template <int LG>
-__device__ __forceinline__ float2 *fft_forward_c(float2 *a, float2 *b, const float2 *twp, int t, int grp)
+__device__ __forceinline__ void filter_pair(const float2 (&in)[Fft<LG>::ITIN][Fft<LG>::IN],
+                                            float2 (&out)[Fft<LG>::ITC][Fft<LG>::NC], float2 *A, float2 *B,
+                                            const float2 *tw, const float *hf, int t, int grp)
 {
-    fft_passes_c<LG, 0>(a, b, twp, t, grp);
-    return a;
-}
-
-// Threads per transform (one radix-16 butterfly each) and groups per CTA.
-__host__ __device__ __forceinline__ int fft_threads(int p)
-{
-    const int t = (p >> 4) > 32 ? (p >> 4) : 32;
-    return t < kFiltThreads ? t : kFiltThreads;
-}
-
-// Shared-memory layout of the filter kernels: twiddle tables, the spectrum
-// Hf (p/2+1 floats), then per group two padded transform buffers.
-struct FiltSmem {
-    int tw_total, hf_floats, group_bytes, groups;
-    __host__ __device__ size_t bytes() const
-    {
-        return (size_t)tw_total * 8 + (size_t)hf_floats * 4 + (size_t)groups * group_bytes;
+    using F = Fft<LG>;
+    constexpr int P = F::P, RL = F::RL, NS = P / RL;  // NS: span and butterflies of the last forward pass
+    float2 *x = A, *y = B;
+    // spectrum product and the inverse's first pass on the outputs X[j + s NS] of the last forward pass
+    auto middle = [&](float2 (&v)[RL], int j) {
+        dft<RL>(v);
+#pragma unroll
+        for (int s2 = 0; s2 < RL; ++s2) {
+            const int k = j + s2 * NS;
+            const float h = hf[k <= (P >> 1) ? k : P - k];
+            v[s2] = make_float2(v[s2].x * h, -v[s2].y * h);  // conj(Z) * Hf
+        }
+        dft<RL>(v);
+    };
+    if constexpr (F::NP > 1) {
+#pragma unroll
+        for (int i = 0; i < F::ITIN; ++i) {
+            const int j = t + i * F::TPF;
+            if ((F::Q1 % F::TPF) != 0 && j >= F::Q1) break;
+            float2 v[16];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) v[r] = in[i][r];
+            dft_half<16>(v);
+            store_butterfly<16, 1>(v, x, j);
+        }
+        group_sync<F::TPF>(grp);
+        forward_passes<LG, 1>(x, y, tw, t, grp);
+        constexpr int ITER = (NS + F::TPF - 1) / F::TPF;
+#pragma unroll(ITER <= 4 ? ITER : 4)
+        for (int i = 0; i < ITER; ++i) {
+            const int j = t + i * F::TPF;
+            if ((NS % F::TPF) != 0 && j >= NS) break;
+            float2 v[RL];
+            load_butterfly<RL, P, NS, false>(v, x, tw + F::fwd_off(F::NP - 1), j);
+            middle(v, j);
+            store_butterfly<RL, 1>(v, y, j);
+        }
+        group_sync<F::TPF>(grp);
+        float2 *z = x;
+        x = y;
+        y = z;
+        inverse_passes<LG, 0>(x, y, tw, t, grp);
+#pragma unroll
+        for (int i = 0; i < F::ITC; ++i) {
+            const int j = t + i * F::TPF;
+            if ((F::QC % F::TPF) != 0 && j >= F::QC) break;
+            float2 v[16];
+            if constexpr (LG == 13)
+                load_butterfly<16, P, P / 16, true>(v, x, tw + F::fwd_off(F::NP - 1), j);
+            else
+                load_butterfly<16, P, P / 16, false>(v, x, tw + F::inv_off(F::NP - 2), j);
+            dft16_low(v);
+#pragma unroll
+            for (int s2 = 0; s2 < 8; ++s2) out[i][s2] = v[s2];
+        }
+    } else {  // p <= 16: one butterfly
+        if (t == 0) {
+            float2 v[RL];
+#pragma unroll
+            for (int r = 0; r < RL / 2; ++r) v[r] = in[0][r];
+            dft_half<RL>(v);
+#pragma unroll
+            for (int s2 = 0; s2 < RL; ++s2) {
+                const float h = hf[s2 <= (P >> 1) ? s2 : P - s2];
+                v[s2] = make_float2(v[s2].x * h, -v[s2].y * h);
+            }
+            dft<RL>(v);
+            store_butterfly<RL, 1>(v, x, 0);
+        }
+        group_sync<F::TPF>(grp);
+        if (t < F::QC) out[0][0] = x[pidx(t)];
+        group_sync<F::TPF>(grp);
     }
-};
-__host__ __device__ inline FiltSmem filt_smem(int p, int tw_total)
-{
-    FiltSmem f;
-    f.tw_total = tw_total;
-    f.hf_floats = ((p / 2 + 1) + 3) & ~3;  // 16-byte multiple
-    f.group_bytes = 2 * padded_len(p) * 8;
-    f.groups = kFiltThreads / fft_threads(p);
-    return f;
-}
-
-template <typename T> __device__ __forceinline__ T store_cvt(float v);
-template <> __device__ __forceinline__ float store_cvt<float>(float v) { return v; }
-template <> __device__ __forceinline__ __half store_cvt<__half>(float v) { return __float2half_rn(v); }
-template <> __device__ __forceinline__ __nv_bfloat16 store_cvt<__nv_bfloat16>(float v)
-{
-    return __float2bfloat16_rn(v);
 }
 
 // Element offset of output row `row` (= b*H + r) of the raw-sample output.
@@ -371,96 +453,112 @@ __device__ __forceinline__ long long out_row_offset(const FiltParams &P, long lo
     return P.out_layout == TK_LAYOUT_SINOGRAM ? ((long long)r * P.L.N + b) * P.Wp : row * (long long)P.Wp;
 }
 
-template <typename T, int LG>
+// Shared memory of the filter kernels: twiddle tables, the spectrum, then per group two transform buffers and the
+// first columns of its warps.
+template <int LG> struct FiltSmem {
+    float2 *tw, *A, *B, *edge;
+    float *hf;
+    __device__ __forceinline__ FiltSmem(float2 *base, int grp)
+    {
+        using F = Fft<LG>;
+        tw = base;
+        hf = reinterpret_cast<float *>(base + F::TW);
+        A = reinterpret_cast<float2 *>(reinterpret_cast<char *>(hf + F::HF) + (size_t)grp * F::group_bytes());
+        B = A + F::P + F::P / 16;
+        edge = B + F::P + F::P / 16;
+    }
+};
+
+// Raw samples of one row at a thread's inputs x = j + r Q1 (0 at x >= W and where not valid), as they are stored
+// (a conversion here would wait for the load).
+template <int LG>
+__device__ __forceinline__ void load_inputs(const LoadParams &L, long long off, bool valid, int t,
+                                            uint32_t (&v)[Fft<LG>::ITIN][Fft<LG>::IN])
+{
+    using F = Fft<LG>;
+#pragma unroll
+    for (int i = 0; i < F::ITIN; ++i)
+#pragma unroll
+        for (int r = 0; r < F::IN; ++r) {
+            const int j = t + i * F::TPF, x = j + r * F::Q1;
+            v[i][r] = 0u;
+            if (valid && j < F::Q1 && x < L.W)
+                v[i][r] = L.input_type == TK_INPUT_U16 ? __ldg(static_cast<const uint16_t *>(L.in) + off + x)
+                                                       : __ldg(static_cast<const uint32_t *>(L.in) + off + x);
+        }
+}
+// Preprocesses both rows' raw samples and packs them.
+template <int LG>
+__device__ __forceinline__ void pack_inputs(const LoadParams &L, int r_a, int r_b, bool valid, bool hasb, int t,
+                                            const uint32_t (&a)[Fft<LG>::ITIN][Fft<LG>::IN],
+                                            const uint32_t (&b)[Fft<LG>::ITIN][Fft<LG>::IN],
+                                            float2 (&in)[Fft<LG>::ITIN][Fft<LG>::IN])
+{
+    using F = Fft<LG>;
+    const float rta = weight_row_term(L, r_a), rtb = weight_row_term(L, r_b);
+    auto value = [&](uint32_t v) { return L.input_type == TK_INPUT_U16 ? (float)v : __uint_as_float(v); };
+#pragma unroll
+    for (int i = 0; i < F::ITIN; ++i)
+#pragma unroll
+        for (int r = 0; r < F::IN; ++r) {
+            const int j = t + i * F::TPF, x = j + r * F::Q1;
+            const bool ok = valid && j < F::Q1 && x < L.W;
+            in[i][r] = ok ? make_float2(pre_from_raw(L, r_a, x, value(a[i][r]), rta),
+                                        hasb ? pre_from_raw(L, r_b, x, value(b[i][r]), rtb) : 0.f)
+                          : make_float2(0.f, 0.f);
+        }
+}
+
+template <int LG>
 __global__ void __launch_bounds__(kFiltThreads) filter_fft_kernel(const __grid_constant__ FiltParams P)
 {
     extern __shared__ __align__(16) float2 fsm[];
-    constexpr int p = 1 << LG;
-    const FFTPlan &pl = P.plan;
-    const FiltSmem lay = filt_smem(p, pl.tw_total);
-    constexpr int TPF = fft_threads_c(p);
-    constexpr int G = kFiltThreads / TPF;
-    const int grp = threadIdx.x / TPF, t = threadIdx.x - grp * TPF;
-    float2 *twp = fsm;
-    float *hf = reinterpret_cast<float *>(fsm + lay.tw_total);
-    float2 *bufA = reinterpret_cast<float2 *>(reinterpret_cast<char *>(hf + lay.hf_floats) + (size_t)grp * lay.group_bytes);
-    float2 *bufB = bufA + padded_len(p);
-    fill_twiddles(twp, pl);
-    for (int k = threadIdx.x; k <= p / 2; k += kFiltThreads) hf[k] = P.Hf[k];
-    const float sigma = P.q_scale ? *P.q_scale : 1.f;
+    using F = Fft<LG>;
+    const int grp = threadIdx.x / F::TPF, t = threadIdx.x - grp * F::TPF;
+    const FiltSmem<LG> S(fsm, grp);
+    fill_twiddles<LG>(S.tw);
+    for (int k = threadIdx.x; k <= F::P / 2; k += kFiltThreads) S.hf[k] = P.Hf[k];
     const int W = P.L.W;
-    T *out = static_cast<T *>(P.out);
+    float *out = static_cast<float *>(P.out);
     __syncthreads();
 
     // Raw samples of a pair group's two rows, fetched one group ahead so that
-    // their latency overlaps the transforms of the current one.  Thread t owns
-    // the run x0 = t NV .. x0 + NV - 1 of each row (NV TPF = p/2 >= W).
-    constexpr int NV = (p / 2 + TPF - 1) / TPF;
-    static_assert(NV * TPF >= p / 2, "sample runs must cover the first half of the transform");
-    const int x0 = t * NV;
-    float raw_a[NV], raw_b[NV];
+    // their latency overlaps the transforms of the current one.
+    uint32_t raw_a[F::ITIN][F::IN], raw_b[F::ITIN][F::IN];
     auto fetch = [&](long long pgf) {
-        const long long pr = pgf * G + grp;
+        const long long pr = pgf * F::G + grp;
         const bool vl = pr < P.npairs;
         const bool hb = vl && 2 * pr + 1 < P.nrows;
         int rr;
         const long long oa = vl ? in_row_offset(P.L, 2 * pr, rr) : 0;
         const long long ob = hb ? in_row_offset(P.L, 2 * pr + 1, rr) : 0;
-        load_run<NV>(P.L, oa, x0, vl, raw_a);
-        load_run<NV>(P.L, ob, x0, hb, raw_b);
+        load_inputs<LG>(P.L, oa, vl, t, raw_a);
+        load_inputs<LG>(P.L, ob, hb, t, raw_b);
     };
-    if ((long long)blockIdx.x * G < P.npairs) fetch(blockIdx.x);
-    for (long long pg = blockIdx.x; pg * G < P.npairs; pg += gridDim.x) {
-        const long long pair = pg * G + grp;
+    if ((long long)blockIdx.x * F::G < P.npairs) fetch(blockIdx.x);
+    for (long long pg = blockIdx.x; pg * F::G < P.npairs; pg += gridDim.x) {
+        const long long pair = pg * F::G + grp;
         const bool valid = pair < P.npairs;
         const long long ra = 2 * pair, rb = 2 * pair + 1;
         const bool hasb = valid && rb < P.nrows;
+        int r_a = 0, r_b = 0;
+        const long long qa = valid ? out_row_offset(P, ra, r_a) : 0, qb = hasb ? out_row_offset(P, rb, r_b) : 0;
+        float2 in[F::ITIN][F::IN], q[F::ITC][F::NC];
+        pack_inputs<LG>(P.L, r_a, r_b, valid, hasb, t, raw_a, raw_b, in);
+        if ((pg + gridDim.x) * F::G < P.npairs) fetch(pg + gridDim.x);
+        filter_pair<LG>(in, q, S.A, S.B, S.tw, S.hf, t, grp);
         if (valid) {
-            int r_a = 0, r_b = 0;
-            in_row_offset(P.L, ra, r_a);
-            if (hasb) in_row_offset(P.L, rb, r_b);
             const float rta = weight_row_term(P.L, r_a), rtb = weight_row_term(P.L, r_b);
 #pragma unroll
-            for (int j = 0; j < NV; ++j) {
-                const int x = x0 + j;
-                if (NV * TPF == p / 2 || x < p / 2)  // short transforms: runs past p/2 are the padding's
-                    bufA[pidx(x)] = x < W ? make_float2(pre_from_raw(P.L, r_a, x, raw_a[j], rta),
-                                                        hasb ? pre_from_raw(P.L, r_b, x, raw_b[j], rtb) : 0.f)
-                                          : make_float2(0.f, 0.f);
-            }
-            for (int x = p / 2 + t; x < p; x += TPF) bufA[pidx(x)] = make_float2(0.f, 0.f);  // zero padding
-        }
-        if ((pg + gridDim.x) * G < P.npairs) fetch(pg + gridDim.x);
-        group_sync<TPF>(grp);
-        float2 *R = fft_forward_c<LG>(bufA, bufB, twp, t, grp);
-        float2 *Sb = (R == bufA) ? bufB : bufA;
-        // conj(Z) * Hf (Hf real and even)
-#pragma unroll 4
-        for (int k = t; k < p; k += TPF) {
-            const float h = hf[k <= (p >> 1) ? k : p - k];
-            const float2 z = R[pidx(k)];
-            R[pidx(k)] = make_float2(z.x * h, -z.y * h);
-        }
-        group_sync<TPF>(grp);
-        float2 *Q = fft_forward_c<LG>(R, Sb, twp, t, grp);
-        if (valid) {
-            int r_a, r_b;
-            T *qa = out + out_row_offset(P, ra, r_a);
-            const float rta = weight_row_term(P.L, r_a);
-            for (int i = t; i < W; i += TPF) {
-                const float w = P.weight_out ? cosine_weight_rt(P.L, rta, i) : 1.f;
-                qa[i] = store_cvt<T>(Q[pidx(i)].x * sigma * w);
-            }
-            if (hasb) {
-                T *qb = out + out_row_offset(P, rb, r_b);
-                const float rtb = weight_row_term(P.L, r_b);
-                for (int i = t; i < W; i += TPF) {
-                    const float w = P.weight_out ? cosine_weight_rt(P.L, rtb, i) : 1.f;
-                    qb[i] = store_cvt<T>(-Q[pidx(i)].y * sigma * w);
+            for (int i = 0; i < F::ITC; ++i)
+#pragma unroll
+                for (int s2 = 0; s2 < F::NC; ++s2) {
+                    const int j = t + i * F::TPF, c = j + s2 * F::QC;
+                    if (j >= F::QC || c >= W) continue;
+                    out[qa + c] = q[i][s2].x * (P.weight_out ? cosine_weight_rt(P.L, rta, c) : 1.f);
+                    if (hasb) out[qb + c] = -q[i][s2].y * (P.weight_out ? cosine_weight_rt(P.L, rtb, c) : 1.f);
                 }
-            }
         }
-        group_sync<TPF>(grp);  // buffers are reused by the next pair group
     }
 }
 
@@ -470,33 +568,30 @@ __global__ void __launch_bounds__(kFiltThreads) filter_fft_kernel(const __grid_c
 // A work unit is RC consecutive detector rows of one projection.  The group
 // filters the unit's rows two at a time (plus the first row of the next unit,
 // which the last coefficient row needs) and keeps the previous filtered row in
-// registers (each thread holds it at the columns of its own entries), so
-// every coefficient row r is formed from filtered rows r and r+1 without
-// another pass over HBM.  Samples outside the detector are 0.
+// registers (each thread holds it at its own columns), so every coefficient
+// row r is formed from filtered rows r and r+1 without another pass over HBM.
+// A thread's columns are j + s QC; column c + 1 sits in the next lane, or, for
+// the last lane of a warp, in the next warp's first columns, which pass through
+// shared memory.  Samples outside the detector are 0.
 
 template <int MODE, int LG>
 __global__ void __launch_bounds__(kFiltThreads) filter_coef_kernel(const __grid_constant__ FiltParams P)
 {
     extern __shared__ __align__(16) float2 fsm[];
-    constexpr int p = 1 << LG;
-    const FFTPlan &pl = P.plan;
-    const FiltSmem lay = filt_smem(p, pl.tw_total);
-    constexpr int TPF = fft_threads_c(p);
-    constexpr int G = kFiltThreads / TPF;
-    const int grp = threadIdx.x / TPF, t = threadIdx.x - grp * TPF;
-    float2 *twp = fsm;
-    float *hf = reinterpret_cast<float *>(fsm + lay.tw_total);
-    float2 *bufA = reinterpret_cast<float2 *>(reinterpret_cast<char *>(hf + lay.hf_floats) + (size_t)grp * lay.group_bytes);
-    float2 *bufB = bufA + padded_len(p);
-    fill_twiddles(twp, pl);
-    for (int k = threadIdx.x; k <= p / 2; k += kFiltThreads) hf[k] = P.Hf[k];
+    using F = Fft<LG>;
+    static_assert(F::ITC == 1 && F::ITIN == 1, "one butterfly per thread (p <= 4096)");
+    constexpr int NC = F::NC;
+    const int grp = threadIdx.x / F::TPF, t = threadIdx.x - grp * F::TPF, lane = threadIdx.x & 31;
+    const FiltSmem<LG> S(fsm, grp);
+    fill_twiddles<LG>(S.tw);
+    for (int k = threadIdx.x; k <= F::P / 2; k += kFiltThreads) S.hf[k] = P.Hf[k];
     const float sigma = P.q_scale ? *P.q_scale : 1.f;
     const int W = P.L.W, H = P.L.H, RC = P.rc;
     const int Wc = MODE == TK_F32_COEF ? W : ((W + 1) & ~1);
     __syncthreads();
 
-    for (long long ug = blockIdx.x; ug * G < P.nunits; ug += gridDim.x) {
-        const long long unit = ug * G + grp;
+    for (long long ug = blockIdx.x; ug * F::G < P.nunits; ug += gridDim.x) {
+        const long long unit = ug * F::G + grp;
         const bool valid = unit < P.nunits;
         const long long b = valid ? unit / P.nchunks : 0;
         const int r0 = valid ? (int)(unit - b * P.nchunks) * RC : 0;
@@ -507,13 +602,9 @@ __global__ void __launch_bounds__(kFiltThreads) filter_coef_kernel(const __grid_
         const int npair = valid ? (rend - r0 + 2) / 2 : 0;
         // every group runs the same number of pair steps
         const int steps = (min(RC, H - 1) + 2) / 2;
-        // Raw samples x0 .. x0 + NV - 1 (x0 = t NV; NV TPF = p/2 >= W) of the
-        // next step's two rows, fetched one step ahead so that their latency
+        // Raw samples of the next step's two rows, fetched one step ahead so that their latency
         // overlaps the transforms.
-        constexpr int NV = (p / 2 + TPF - 1) / TPF;
-        static_assert(NV * TPF >= p / 2, "sample runs must cover the first half of the transform");
-        const int x0 = t * NV;
-        float raw_a[NV], raw_b[NV];
+        uint32_t raw_a[1][F::IN], raw_b[1][F::IN];
         auto fetch = [&](int kk) {
             const bool lv = valid && kk < npair;
             const int qa = r0 + 2 * kk, qb = qa + 1;
@@ -521,76 +612,56 @@ __global__ void __launch_bounds__(kFiltThreads) filter_coef_kernel(const __grid_
             int rr;
             const long long oa = lv ? in_row_offset(P.L, bf * H + qa, rr) : 0;
             const long long ob = hb ? in_row_offset(P.L, bf * H + qb, rr) : 0;
-            load_run<NV>(P.L, oa, x0, lv, raw_a);
-            load_run<NV>(P.L, ob, x0, hb, raw_b);
+            load_inputs<LG>(P.L, oa, lv, t, raw_a);
+            load_inputs<LG>(P.L, ob, hb, t, raw_b);
         };
-        // The previous filtered row (ra - 1) at the columns c, c+1, c+2 of
-        // this thread's column pairs c = 2 (i TPF + t): carried in registers
-        // from one step to the next.
-        constexpr int NPR = NV / 2 > 0 ? NV / 2 : 1;
-        float pv[NPR][3];
+        float pq[NC], pd[NC];  // the previous filtered row (ra - 1) at this thread's columns: value, difference to c + 1
 #pragma unroll
-        for (int i = 0; i < NPR; ++i) pv[i][0] = pv[i][1] = pv[i][2] = 0.f;
+        for (int s2 = 0; s2 < NC; ++s2) pq[s2] = pd[s2] = 0.f;
         fetch(0);
         for (int k = 0; k < steps; ++k) {
             const bool live = valid && k < npair;
             const int ra = r0 + 2 * k, rb = ra + 1;
             const bool hasb = live && rb <= rend;
-            if (live) {
-                const float rta = weight_row_term(P.L, ra), rtb = weight_row_term(P.L, rb);
-#pragma unroll
-                for (int j = 0; j < NV; ++j) {
-                    const int x = x0 + j;
-                    if (NV * TPF == p / 2 || x < p / 2)  // short transforms: runs past p/2 are the padding's
-                        bufA[pidx(x)] = x < W ? make_float2(pre_from_raw(P.L, ra, x, raw_a[j], rta),
-                                                            hasb ? pre_from_raw(P.L, rb, x, raw_b[j], rtb) : 0.f)
-                                              : make_float2(0.f, 0.f);
-                }
-                for (int x = p / 2 + t; x < p; x += TPF) bufA[pidx(x)] = make_float2(0.f, 0.f);  // zero padding
-            }
+            float2 in[1][F::IN], q[1][NC];
+            pack_inputs<LG>(P.L, ra, rb, live, hasb, t, raw_a, raw_b, in);
             if (k + 1 < steps) fetch(k + 1);
-            group_sync<TPF>(grp);
-            float2 *R = fft_forward_c<LG>(bufA, bufB, twp, t, grp);
-            float2 *Sb = (R == bufA) ? bufB : bufA;
-#pragma unroll 4
-            for (int kk = t; kk < p; kk += TPF) {
-                const float h = hf[kk <= (p >> 1) ? kk : p - kk];
-                const float2 z = R[pidx(kk)];
-                R[pidx(kk)] = make_float2(z.x * h, -z.y * h);
+            filter_pair<LG>(in, q, S.A, S.B, S.tw, S.hf, t, grp);
+            // rows ra (x) and rb (y); columns past W read as 0
+#pragma unroll
+            for (int s2 = 0; s2 < NC; ++s2) {
+                const bool in_row = t < F::QC && t + s2 * F::QC < W;
+                q[0][s2] = in_row ? make_float2(q[0][s2].x * sigma, hasb ? -q[0][s2].y * sigma : 0.f)
+                                  : make_float2(0.f, 0.f);
             }
-            group_sync<TPF>(grp);
-            const float2 *Q = fft_forward_c<LG>(R, Sb, twp, t, grp);
-            if (live) {
-                const size_t base = (size_t)bf * H;
-                const float zero[3] = {0.f, 0.f, 0.f};
+            if (lane == 0) {
 #pragma unroll
-                for (int i = 0; i < NPR; ++i) {
-                    const int c = 2 * (i * TPF + t);
-                    if (c < W) {
-                        // rows ra (Re) and rb (-Im) at c, c+1, c+2; columns >= W read as 0
-                        float a[3], bb[3];
+                for (int s2 = 0; s2 < NC; ++s2) S.edge[(t >> 5) * (NC + 1) + s2] = q[0][s2];
+            }
+            group_sync<F::TPF>(grp);
+            const bool last = t == F::QC - 1;  // its next column is the first of the next s
+            const float2 *edge = S.edge + (last ? 1 : ((t >> 5) + 1) * (NC + 1));
+            const size_t base = ((size_t)bf * H + ra) * Wc;
 #pragma unroll
-                        for (int k3 = 0; k3 < 3; ++k3) {
-                            const float2 q = Q[pidx(c + k3)];
-                            const bool in = c + k3 < W;
-                            a[k3] = in ? q.x * sigma : 0.f;
-                            bb[k3] = in ? -q.y * sigma : 0.f;
-                        }
-                        if (ra - 1 >= r0)  // prev = row ra-1, next = row ra
-                            emit_coef_pair<MODE>(P.out, (base + ra - 1) * Wc, c, W, pv[i], a);
-                        if (ra < r1)  // next = row rb, or 0 below the detector's last row
-                            emit_coef_pair<MODE>(P.out, (base + ra) * Wc, c, W, a, hasb ? bb : zero);
-                        if (hasb && rb < r1 && rb == rend)  // detector's last row, nothing follows
-                            emit_coef_pair<MODE>(P.out, (base + rb) * Wc, c, W, bb, zero);
-                        if (hasb) {
-                            pv[i][0] = bb[0];
-                            pv[i][1] = bb[1];
-                            pv[i][2] = bb[2];
-                        }
-                    }
+            for (int s2 = 0; s2 < NC; ++s2) {
+                const int c = t + s2 * F::QC;
+                const float2 v = q[0][s2];
+                float2 n;
+                n.x = __shfl_down_sync(0xffffffffu, v.x, 1);
+                n.y = __shfl_down_sync(0xffffffffu, v.y, 1);
+                if (last || lane == 31) n = c + 1 < W ? edge[s2] : make_float2(0.f, 0.f);
+                const float da = n.x - v.x, db = n.y - v.y;
+                if (live && t < F::QC && c < Wc) {
+                    if (ra - 1 >= r0)  // the previous row, followed by row ra
+                        store_coef<MODE>(P.out, base - Wc + c, pq[s2], pd[s2], v.x - pq[s2], da - pd[s2]);
+                    if (ra < r1)  // followed by row rb, or 0 below the detector's last row
+                        store_coef<MODE>(P.out, base + c, v.x, da, v.y - v.x, db - da);
+                    if (hasb && rb < r1 && rb == rend)  // detector's last row, nothing follows
+                        store_coef<MODE>(P.out, base + Wc + c, v.y, db, 0.f - v.y, 0.f - db);
                 }
+                pq[s2] = v.y;
+                pd[s2] = db;
             }
-            group_sync<TPF>(grp);  // the buffers are rewritten by the next step
         }
     }
 }
@@ -711,20 +782,28 @@ static const Spectrum &spectrum(int W, float tau, int window, int p)
 
 // The kernel instantiated for storage `precision` and pad length 2^lg
 // (2 <= lg <= 13; coefficient storage up to lg = 12, i.e. W <= 2048).
-template <int LG> static const void *filter_kernel_lg(int precision)
+struct FiltKernel {
+    const void *fn = nullptr;
+    size_t smem = 0;
+    int groups = 1;
+};
+template <int LG> static FiltKernel filter_kernel_lg(int precision)
 {
+    FiltKernel k;
+    k.smem = Fft<LG>::smem();
+    k.groups = Fft<LG>::G;
     switch (precision) {
-    case TK_F32: return reinterpret_cast<const void *>(&filter_fft_kernel<float, LG>);
-    case TK_F16: if constexpr (LG <= 12) return reinterpret_cast<const void *>(&filter_coef_kernel<TK_F16, LG>); break;
-    case TK_BF16: if constexpr (LG <= 12) return reinterpret_cast<const void *>(&filter_coef_kernel<TK_BF16, LG>); break;
+    case TK_F32: k.fn = reinterpret_cast<const void *>(&filter_fft_kernel<LG>); break;
+    case TK_F16: if constexpr (LG <= 12) k.fn = reinterpret_cast<const void *>(&filter_coef_kernel<TK_F16, LG>); break;
+    case TK_BF16: if constexpr (LG <= 12) k.fn = reinterpret_cast<const void *>(&filter_coef_kernel<TK_BF16, LG>); break;
     case TK_F32_COEF:
-        if constexpr (LG <= 12) return reinterpret_cast<const void *>(&filter_coef_kernel<TK_F32_COEF, LG>);
+        if constexpr (LG <= 12) k.fn = reinterpret_cast<const void *>(&filter_coef_kernel<TK_F32_COEF, LG>);
         break;
     }
-    return nullptr;
+    return k;
 }
 
-static const void *filter_kernel_fn(int precision, int lg)
+static FiltKernel filter_kernel(int precision, int lg)
 {
     switch (lg) {
     case 2: return filter_kernel_lg<2>(precision);
@@ -740,15 +819,36 @@ static const void *filter_kernel_fn(int precision, int lg)
     case 12: return filter_kernel_lg<12>(precision);
     case 13: return filter_kernel_lg<13>(precision);
     }
-    return nullptr;
+    return FiltKernel{};
 }
 
-static int launch_filter_typed(const FiltParams &P, int p, cudaStream_t stream, int precision)
+// Rows per work unit of a coefficient image: each of the `slots` resident groups takes ceil(units / slots) units of
+// (rc + 2) / 2 pair steps (the first row of the next unit is filtered too), so unit sizes that leave the last round
+// nearly empty cost up to a round.  Picks the number of units per projection with the fewest steps; 90 x 1024 rows on
+// 608 groups: 54 rows, 84 steps, against 64 rows, 99 steps (that filter 668 -> 622 us).
+static int rows_per_unit(int N, int H, long long slots)
 {
-    const void *fn = filter_kernel_fn(precision, P.lg);
+    long long best = -1;
+    int rc = 64;
+    for (int n = 1; n <= std::max(1, H / 8); ++n) {
+        const int r = ((H + n - 1) / n + 1) & ~1;  // even: the same row pairs whatever the unit
+        const long long units = (long long)N * ((H + r - 1) / r);
+        const long long cost = (units + slots - 1) / slots * ((std::min(r, H - 1) + 2) / 2);
+        if (best < 0 || cost < best) {
+            best = cost;
+            rc = r;
+        }
+    }
+    return rc;
+}
+
+static int launch_filter_typed(FiltParams &P, int p, cudaStream_t stream, int precision)
+{
+    const FiltKernel k = filter_kernel(precision, P.lg);
+    const void *fn = k.fn;
     TK_CHECK(fn, TK_ERR_UNSUPPORTED, "filter: no kernel for pad length %d with this storage", p);
-    const int G = kFiltThreads / fft_threads(p);
-    const size_t smem = filt_smem(p, P.plan.tw_total).bytes();
+    const int G = k.groups;
+    const size_t smem = k.smem;
     TK_CHECK(smem <= 227 * 1024, TK_ERR_UNSUPPORTED, "filter: pad length %d needs too much shared memory", p);
     TK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int dev = 0, sms = 0, per_sm = 0;
@@ -756,10 +856,15 @@ static int launch_filter_typed(const FiltParams &P, int p, cudaStream_t stream, 
     TK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     TK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kFiltThreads, smem));
     if (per_sm < 1) per_sm = 1;
+    if (is_coef(precision)) {
+        P.rc = rows_per_unit(P.L.N, P.L.H, (long long)sms * per_sm * G);
+        P.nchunks = (P.L.H + P.rc - 1) / P.rc;
+        P.nunits = (long long)P.L.N * P.nchunks;
+    }
     const long long work = is_coef(precision) ? P.nunits : P.npairs;
     const long long groups = (work + G - 1) / G;
     const long long grid = std::min<long long>(groups, (long long)sms * per_sm);
-    void *args[] = {const_cast<FiltParams *>(&P)};
+    void *args[] = {&P};
     TK_CUDA(cudaLaunchKernel(fn, dim3((unsigned)std::max<long long>(grid, 1)), dim3(kFiltThreads), args, smem,
                              stream));
     count_launch();
@@ -827,11 +932,7 @@ int launch_filter(const tk_geometry &g, const void *d_in, int input_type, int la
     int lg = 0;
     while ((1 << lg) < p) ++lg;
     P.lg = lg;
-    P.plan = fft_plan(lg);
     P.precision = precision;
-    P.rc = 64;
-    P.nchunks = (g.H + P.rc - 1) / P.rc;
-    P.nunits = (long long)g.N * P.nchunks;
     P.fgrp = fgrp > 0 ? fgrp : 0;
     P.fstride = fgrp > 0 ? fstride : 0;
     std::memcpy(P.Hf, sp.Hf.data(), sizeof(float) * sp.Hf.size());
@@ -936,7 +1037,6 @@ int launch_filter_transpose(const tk_geometry &g, const float *d_qbar, int windo
     int lg = 0;
     while ((1 << lg) < p) ++lg;
     P.lg = lg;
-    P.plan = fft_plan(lg);
     P.precision = TK_F32;
     std::memcpy(P.Hf, sp.Hf.data(), sizeof(float) * sp.Hf.size());
     return launch_filter_typed(P, p, stream, TK_F32);

@@ -115,6 +115,23 @@ __device__ __forceinline__ void emit_coef_pair(void *img, size_t row_base, int c
     }
 }
 
+// One coefficient entry (see tk_precision) at entry offset `at`.
+template <int MODE>
+__device__ __forceinline__ void store_coef(void *img, size_t at, float Q, float dU, float dV, float dUV)
+{
+    if constexpr (MODE == TK_F32_COEF) {
+        static_cast<float4 *>(img)[at] = make_float4(Q, dU, dV, dUV);
+    } else if constexpr (MODE == TK_F16) {
+        const __half2 l = __floats2half2_rn(Q, dV), h = __floats2half2_rn(dU, dUV);
+        static_cast<uint2 *>(img)[at] =
+            make_uint2(*reinterpret_cast<const uint32_t *>(&l), *reinterpret_cast<const uint32_t *>(&h));
+    } else {
+        const __nv_bfloat162 l = __floats2bfloat162_rn(Q, dV), h = __floats2bfloat162_rn(dU, dUV);
+        static_cast<uint2 *>(img)[at] =
+            make_uint2(*reinterpret_cast<const uint32_t *>(&l), *reinterpret_cast<const uint32_t *>(&h));
+    }
+}
+
 // Derived load parameters: D^2, the scalar flat-field reciprocal, and whether
 // rows can be read in 16-byte chunks (aligned base, row pitch a multiple of
 // 16 bytes, so every chunk that starts below W lies inside its row).
