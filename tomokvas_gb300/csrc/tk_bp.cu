@@ -186,7 +186,12 @@ __device__ __forceinline__ void direct_update(uint32_t sbase, uint32_t row_bytes
 // ---------------------------------------------------------------------------
 // Direct FP32 backprojector: bilinear gathers straight from the staged
 // sample tile (four LDS.32 per update).
-template <typename S, int TX, int TY, int TZ, int STAGES, int MINB, bool PACKED = false>
+//
+// A step takes NB projections: their column geometries (a divide and the trig
+// load each) are formed together before the first stage's wait, and one
+// barrier and one refill serve the NB stages.  (Forming the box positions and
+// checks there too, with all waits before all updates, measured 1.4 % slower.)
+template <typename S, int TX, int TY, int TZ, int STAGES, int MINB, bool PACKED, int NB>
 __global__ void __launch_bounds__(TX *TY, MINB)
     bp_tma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ BPParams P)
 {
@@ -250,20 +255,29 @@ __global__ void __launch_bounds__(TX *TY, MINB)
 
     const float cZ = P.cZ, Hm1 = P.Hm1;
     const uint32_t row_bytes = (uint32_t)P.BW * 4u, smem0 = smem_u32(smem);
+    static_assert(STAGES % NB == 0, "a step's stages are consecutive");
     int b = 0;
-    for (; b < P.N; ++b) {
-        const int s = b % STAGES;
-        const uint32_t parity = (uint32_t)(b / STAGES) & 1u;
-        float U, u;
-        column_geometry(aX, aY, P.trig[b], P.D, P.cX, U, u);  // before the wait: a divide and the trig load
-        const bool got = mbar_wait_bounded(&full[s], parity, kWaitLimitNs);
-        if (!got) {
-            atomicOr(P.err, ERR_WAIT_TIMEOUT);
-            s_abort = 1;
+    for (; b < P.N; b += NB) {
+        float Us[NB], us[NB];
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            Us[i] = us[i] = 0.f;
+            if (b + i < P.N) column_geometry(aX, aY, P.trig[b + i], P.D, P.cX, Us[i], us[i]);
         }
-        const int bx0 = boxo[b].x, by0 = boxo[b].y;
-        if (active && got) {
-            if (u >= 0.f && u <= P.Wm1) {  // column inside the detector (kernel.cu:127-128)
+        const int s0 = b % STAGES;
+        const uint32_t parity = (uint32_t)(b / STAGES) & 1u;
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            if (b + i >= P.N) break;
+            const int s = s0 + i;
+            const bool got = mbar_wait_bounded(&full[s], parity, kWaitLimitNs);
+            if (!got) {
+                atomicOr(P.err, ERR_WAIT_TIMEOUT);
+                s_abort = 1;
+            }
+            const int bx0 = boxo[b + i].x, by0 = boxo[b + i].y;
+            const float U = Us[i], u = us[i];
+            if (active && got && u >= 0.f && u <= P.Wm1) {  // column inside the detector (kernel.cu:127-128)
                 const float U2 = __fmul_rn(U, U);
                 const float fla = __fadd_rd(u, kMagic);
                 const int a = __float_as_int(fla) - kMagicBits;
@@ -285,12 +299,16 @@ __global__ void __launch_bounds__(TX *TY, MINB)
                 }
             }
         }
-        __syncthreads();  // every thread is done with stage s
+        __syncthreads();  // every thread is done with the step's stages
         if (s_abort) break;
-        if (tid == 0 && b + STAGES < P.N) {
-            mbar_arrive_expect_tx(&full[s], stage_bytes);
-            tma_load_3d(stages + (size_t)s * P.stage_elems, &tmap, boxo[b + STAGES].x, boxo[b + STAGES].y,
-                        b + STAGES, &full[s]);
+        if (tid == 0) {
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                const int k = b + i + STAGES;
+                if (k >= P.N) break;
+                mbar_arrive_expect_tx(&full[s0 + i], stage_bytes);
+                tma_load_3d(stages + (size_t)(s0 + i) * P.stage_elems, &tmap, boxo[k].x, boxo[k].y, k, &full[s0 + i]);
+            }
         }
     }
 
@@ -1546,15 +1564,16 @@ struct BPVariant {
     const char *name;
     int qcap = 0;  // > 0: bp_quad_kernel with staged boxes of up to qcap bytes (needs quad_eligible)
     bool qauto = false;  // a quarter-turn variant the default selection tries, in table order
+    bool zsplit = false;  // fewer slices per tile than the format's default: taken for small volumes (same bits)
 };
 
 
 #define TK_BP_DIRECT(TX, TY, TZ, ST) \
-    {reinterpret_cast<const void *>(&bp_tma_kernel<StoreF32, TX, TY, TZ, ST, 2>), nullptr, TK_F32, TX, TY, TZ, ST, \
-     false, "direct<f32," #TX "," #TY "," #TZ "," #ST ">"}
-#define TK_BP_DIRECT_PK(TX, TY, TZ, ST) \
-    {reinterpret_cast<const void *>(&bp_tma_kernel<StoreF32, TX, TY, TZ, ST, 2, true>), nullptr, TK_F32, TX, TY, TZ, \
-     ST, false, "direct_x2<f32," #TX "," #TY "," #TZ "," #ST ">"}
+    {reinterpret_cast<const void *>(&bp_tma_kernel<StoreF32, TX, TY, TZ, ST, 2, false, 1>), nullptr, TK_F32, TX, TY, \
+     TZ, ST, false, "direct<f32," #TX "," #TY "," #TZ "," #ST ">"}
+#define TK_BP_DIRECT_PK(TX, TY, TZ, ST, MB, NB, ZS) \
+    {reinterpret_cast<const void *>(&bp_tma_kernel<StoreF32, TX, TY, TZ, ST, MB, true, NB>), nullptr, TK_F32, TX, TY, \
+     TZ, ST, false, "direct_x2<f32," #TX "," #TY "," #TZ "," #ST ">", 0, false, ZS}
 #define TK_BP_CIMG(P, PN, TX, TY, TZ, ST, MB) \
     {reinterpret_cast<const void *>(&bp_cimg_kernel<P, TX, TY, TZ, ST, false, MB>), \
      reinterpret_cast<const void *>(&bp_cimg_kernel<P, TX, TY, TZ, ST, true, MB>), P, TX, TY, TZ, ST, true, \
@@ -1595,7 +1614,7 @@ struct BPVariant {
 // the quarter-turn kernel with 16 x 8 tiles, else walk 4.  The half-math
 // walks (FP16 interpolation arithmetic) are selectable only.
 static const BPVariant kVariants[] = {
-    TK_BP_DIRECT_PK(16, 16, 32, 4),
+    TK_BP_DIRECT_PK(16, 16, 32, 4, 2, 2, false),
     TK_BP_QUADF(TK_F16, "f16", 6144, 2, true, 8),
     TK_BP_CIMG_F(TK_F16, "f16", 16, 16, 64, 3, 2),
     TK_BP_QUADF(TK_BF16, "bf16", 6144, 2, true, 8),
@@ -1626,6 +1645,9 @@ static const BPVariant kVariants[] = {
     TK_BP_CIMG_PK(TK_F16, "f16", 16, 16, 48, 3, 2),
     TK_BP_CIMG(TK_F32_COEF, "f32c", 16, 16, 32, 3, 2),
     TK_BP_CIMG(TK_F32_COEF, "f32c", 16, 16, 32, 2, 3),
+    // few slices per tile for small FP32 volumes (z_split)
+    TK_BP_DIRECT_PK(16, 16, 8, 12, 4, 4, true),
+    TK_BP_DIRECT_PK(16, 16, 4, 8, 4, 4, true),
     // two-stage twins of the 16-bit general walks, taken where three staged boxes would leave
     // room for one CTA per SM only (two_stage_twin)
     TK_BP_CIMG_F(TK_F16, "f16", 16, 16, 64, 2, 2),
@@ -1657,6 +1679,24 @@ static const BPVariant *two_stage_twin(const BPVariant *v)
             c.name[np] == '<')
             return &c;
     return nullptr;
+}
+
+// The FP32 variant for `columns` tiles per slice layer and nz slices: the default (32 slices per tile), or the same
+// walk with 8 or 4, where tiles of 32 would leave SMs idle or walk slices past the end.  Estimates of the time per 96
+// projections in us from x CTAs per SM, fitted to cubes of 32 to 256 and to slabs: 32 slices max(108, 55 + 65 x),
+// 8 slices 40 + 19.5 x, 4 slices 25 + 14.2 x (a step's geometry, wait and barrier cost about three slices).
+// Measured, 32 / 8 / 4 slices: 64^2 x 48 109 / 54 / 53 us, 80^2 x 64 109 / 68 / 63, 96^3 132 / 94 / 123, 128^3
+// 191 / 181 / 223, 160^3 277 / 299 / 390, 512^2 x 16 430 / 288 / 373.
+static const BPVariant *z_split(const BPVariant *v, long long columns, int nz, int sms)
+{
+    auto cost = [&](int TZ) {
+        const double x = (double)(columns * ((nz + TZ - 1) / TZ)) / sms;
+        return TZ == 32 ? std::max(108.0, 55.0 + 65.0 * x) : TZ == 8 ? 40.0 + 19.5 * x : 25.0 + 14.2 * x;
+    };
+    const BPVariant *best = v;
+    for (const auto &c : kVariants)
+        if (c.zsplit && c.precision == v->precision && cost(c.TZ) < cost(best->TZ)) best = &c;
+    return best;
 }
 
 // Analytic bound of a tile's footprint extent (see the derivation in the
@@ -1765,6 +1805,12 @@ static int launch_bp_impl(const tk_geometry &g, const void *d_q, int precision, 
         TK_CHECK(v, TK_ERR_INVALID, "backproject: no general variant for precision %d", precision);
     }
     const bool quad = v->qcap > 0;
+    if (precision == TK_F32 && g_variant_override < 0) {
+        int dev = 0, sms = 0;
+        TK_CUDA(cudaGetDevice(&dev));
+        TK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        v = z_split(v, (long long)((g.X + v->TX - 1) / v->TX) * ((g.Y + v->TY - 1) / v->TY), nz, sms);
+    }
     auto encode = get_encode_fn();
     TK_CHECK(encode, TK_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
 
