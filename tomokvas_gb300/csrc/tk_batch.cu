@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     volatile int *ctl = reinterpret_cast<volatile int *>(full + STAGES);  // [0] unit, [1] abort
 
     const int tid = threadIdx.x;
-    const int tx = tid % TX, ty = tid / TX;
+    const int tx = tile_xy<TX>(tid).x, ty = tile_xy<TX>(tid).y;
     const uint32_t smem0 = smem_u32(smem);
     if (tid == 0) {
         ctl[1] = 0;

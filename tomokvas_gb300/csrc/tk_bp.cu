@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     volatile int &s_abort = *reinterpret_cast<int *>(full + STAGES);
 
     const int tid = threadIdx.x;
-    const int tx = tid % TX, ty = tid / TX;
+    const int tx = tile_xy<TX>(tid).x, ty = tile_xy<TX>(tid).y;
     const int2 tile = tile_of(blockIdx.x, P.tilesX, P.tilesY);
     const int x0 = tile.x * TX, y0 = tile.y * TY;
     const int z0 = blockIdx.y * TZ;
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     volatile int &s_abort = *reinterpret_cast<int *>(full + STAGES);
 
     const int tid = threadIdx.x;
-    const int tx = tid % TX, ty = tid / TX;
+    const int tx = tile_xy<TX>(tid).x, ty = tile_xy<TX>(tid).y;
     const int2 tile = tile_of(blockIdx.x, P.tilesX, P.tilesY);
     const int x0 = tile.x * TX, y0 = tile.y * TY;
     // Full chunks of TZ slices.  16-bit storage: the last chunk, when fewer than
@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(16 * TYQ, (PREC == TK_F32_COEF ? 2 : 32 / TYQ)
     int *s_issued = reinterpret_cast<int *>(full + STAGES) + 1;  // steps issued so far
 
     const int tid = threadIdx.x;
-    const int lx = tid % TX, ly = tid / TX;
+    const int lx = tile_xy<TX>(tid).x, ly = tile_xy<TX>(tid).y;
     const int2 tile = tile_of(blockIdx.x, P.tilesX / 2, P.tilesY / 2);  // a tile of the first quadrant
     const int x0 = tile.x * TX, y0 = tile.y * TY;
     const int zc = blockIdx.y * TZ;

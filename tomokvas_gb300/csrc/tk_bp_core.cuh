@@ -26,6 +26,22 @@ __device__ __forceinline__ int2 tile_of(int i, int tilesX, int tilesY)
     return make_int2(g * kTileGroup + r % w, r / w);
 }
 
+// Column (x, y) of thread tid in a tile TX columns wide: a warp covers 8 x 4
+// columns, each half of it 4 x 4, each quarter 4 x 2, each eighth 2 x 2.  The
+// columns that one shared-memory phase reads (a half warp for 8-byte entries, a
+// quarter for 16-byte ones) then span few detector columns and, nearly always,
+// one row, so they rarely share a bank; with 16 columns of one tile row in a
+// half warp, a scale above 1 spreads them past the 16 entries of a phase and the
+// rows drift apart.  48 slices of 640^2 at scale 1.1 with FP32 coefficients
+// 2569 -> 2327 us, 256^3 FP32 samples 1719 -> 1692, 1024^3 FP16 by quarter turns
+// 258.7 -> 256.6 ms (8 x 2 halves: 2567 us, 1693 us, 257.1 ms).
+template <int TX> __device__ __forceinline__ int2 tile_xy(int tid)
+{
+    const int w = tid >> 5, l = tid & 31;
+    const int x = (l & 1) | ((l >> 1) & 2) | ((l >> 2) & 4), y = ((l >> 1) & 1) | ((l >> 2) & 2);
+    return make_int2((w % (TX / 8)) * 8 + x, (w / (TX / 8)) * 4 + y);
+}
+
 // Per column-angle geometry with every rounding spelled out:
 //   S = aX cos + aY sin,  T = aY cos - aX sin,  U = D / (D - S),  u = T U + cX
 // (kernel.cu:102-109).  Every kernel evaluates it through this function --
