@@ -19,7 +19,8 @@ struct LoadParams {
     float cX, cZ, D;
     float D2;       // D * D
     float inv_den;  // 1 / max(flat - dark, floor) for scalar flat/dark
-    int vec;        // rows start 16-byte aligned and span whole 16-byte chunks: chunked loads
+    int gran;       // rows start aligned to and span whole units of 16, 8 or 4 bytes; 0: none of these
+    int map_vec;    // dark and flat rows start 16-byte aligned and span whole 16-byte chunks
 };
 
 // Element offset of the first sample of output row `row` (= b*H + r) in the input.
@@ -56,6 +57,30 @@ __device__ __forceinline__ float load_raw(const LoadParams &L, long long off, in
 // den = max(flat - dark, floor); here in FP32 with __logf, absolute error
 // below 4e-7 for transmissions near 1), then the cosine weight (kernel.cu:
 // 195-199).  rt is the row's weight_row_term.
+__host__ __device__ __forceinline__ bool has_maps(const LoadParams &L)
+{
+    return L.input_type == TK_INPUT_U16 && (L.dark || L.flat);
+}
+// Transmission -> line integral, weighted.
+__device__ __forceinline__ float pre_finish(const LoadParams &L, int x, float t, float rt)
+{
+    float val = fmaf(L.A, __logf(t), L.B);
+    if (L.invert) val = -val;
+    return L.weight_in ? val * cosine_weight_rt(L, rt, x) : val;
+}
+// With maps: dk and fl are the pixel's dark and flat.
+__device__ __forceinline__ float pre_maps(const LoadParams &L, int x, float raw, float dk, float fl, float rt)
+{
+    return pre_finish(L, x, __fdividef(fmaxf(raw - dk, L.floor_counts), fmaxf(fl - dk, L.floor_counts)), rt);
+}
+// Without: FP32 line integrals, or counts with a scalar dark and flat.
+__device__ __forceinline__ float pre_scalar(const LoadParams &L, int x, float raw, float rt)
+{
+    if (L.input_type == TK_INPUT_U16)
+        return pre_finish(L, x, fmaxf(raw - L.dark_v, L.floor_counts) * L.inv_den, rt);
+    return L.weight_in ? raw * cosine_weight_rt(L, rt, x) : raw;
+}
+// Either, one sample with its own loads.
 __device__ __forceinline__ float pre_from_raw(const LoadParams &L, int r, int x, float raw, float rt)
 {
     float val = raw;
@@ -75,11 +100,41 @@ __device__ __forceinline__ float pre_from_raw(const LoadParams &L, int r, int x,
     if (!L.weight_in) return val;
     return val * cosine_weight_rt(L, rt, x);
 }
-
-// Preprocessed (log if raw, cosine weighted) sample x of a row.
-__device__ __forceinline__ float load_pre(const LoadParams &L, long long off, int r, int x)
+// Dark and flat of the pixels x0, x0 + step, ... of row r (N of them, those below W).  A caller loads a run of
+// them before it uses the first: one by one, each sample would wait for its own two loads.
+template <int N>
+__device__ __forceinline__ void load_maps(const LoadParams &L, int r, int x0, int step, float (&dk)[N], float (&fl)[N])
 {
-    return pre_from_raw(L, r, x, load_raw(L, off, x), weight_row_term(L, r));
+    const size_t row = (size_t)r * L.W;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int x = x0 + i * step;
+        dk[i] = L.dark && x < L.W ? __ldg(L.dark + row + x) : L.dark_v;
+        fl[i] = L.flat && x < L.W ? __ldg(L.flat + row + x) : L.flat_v;
+    }
+}
+// Preprocesses the eight counts x0 .. x0 + 7 (x0 a multiple of 8, below W) of row r in place, with maps, which are
+// read four pixels at a time, in 16-byte loads where they allow it; samples at or past W become 0.
+__device__ __forceinline__ void pre8_maps(const LoadParams &L, int r, int x0, float rt, float (&v)[8])
+{
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+        float dk[4], fl[4];
+        if (L.map_vec && x0 + h < L.W) {
+            const size_t at = (size_t)r * L.W + x0 + h;
+            const float4 d = L.dark ? __ldg(reinterpret_cast<const float4 *>(L.dark + at))
+                                    : make_float4(L.dark_v, L.dark_v, L.dark_v, L.dark_v);
+            const float4 f = L.flat ? __ldg(reinterpret_cast<const float4 *>(L.flat + at))
+                                    : make_float4(L.flat_v, L.flat_v, L.flat_v, L.flat_v);
+            dk[0] = d.x, dk[1] = d.y, dk[2] = d.z, dk[3] = d.w;
+            fl[0] = f.x, fl[1] = f.y, fl[2] = f.z, fl[3] = f.w;
+        } else {
+            load_maps<4>(L, r, x0 + h, 1, dk, fl);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            v[h + e] = x0 + h + e < L.W ? pre_maps(L, x0 + h + e, v[h + e], dk[e], fl[e], rt) : 0.f;
+    }
 }
 
 // Coefficient entries of columns c and c+1 of one row (c even, c < W) from
@@ -132,9 +187,9 @@ __device__ __forceinline__ void store_coef(void *img, size_t at, float Q, float 
     }
 }
 
-// Derived load parameters: D^2, the scalar flat-field reciprocal, and whether
-// rows can be read in 16-byte chunks (aligned base, row pitch a multiple of
-// 16 bytes, so every chunk that starts below W lies inside its row).
+// Derived load parameters: D^2, the scalar flat-field reciprocal, and the
+// largest unit that rows can be read in (aligned base, row pitch a multiple of
+// it, so every unit that starts below W lies inside its row).
 inline void finish_load_params(LoadParams &L)
 {
     L.D2 = L.D * L.D;
@@ -142,7 +197,11 @@ inline void finish_load_params(LoadParams &L)
     if (L.input_type == TK_INPUT_U16 && !L.dark && !L.flat)
         L.inv_den = 1.f / std::fmax(L.flat_v - L.dark_v, L.floor_counts);
     const int es = L.input_type == TK_INPUT_U16 ? 2 : 4;
-    L.vec = (reinterpret_cast<uintptr_t>(L.in) % 16 == 0) && ((long long)L.in_pitch * es) % 16 == 0;
+    L.gran = 0;
+    for (int b = 16; b >= 4 && !L.gran; b /= 2)
+        if (reinterpret_cast<uintptr_t>(L.in) % b == 0 && ((long long)L.in_pitch * es) % b == 0) L.gran = b;
+    L.map_vec = L.W % 4 == 0 && reinterpret_cast<uintptr_t>(L.dark) % 16 == 0 &&
+                reinterpret_cast<uintptr_t>(L.flat) % 16 == 0;
 }
 
 }  // namespace tk

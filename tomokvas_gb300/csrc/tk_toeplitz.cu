@@ -154,28 +154,11 @@ __device__ __forceinline__ void split_bf16x2(float a, float b, uint32_t &hi, uin
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
-// Raw samples j0 .. j0+7 (j0 a multiple of 8) of the row at element offset off; 0 at or past W.
+// Raw samples j0 .. j0+7 of the row at element offset off; 0 at or past W.
 __device__ __forceinline__ void load8(const LoadParams &L, long long off, int j0, float (&v)[8])
 {
-    if (L.vec && L.input_type == TK_INPUT_U16) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(L.in) + off + j0));
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {  // count c as (2^23 + c) - 2^23: exact, no integer-to-float conversion
-            v[2 * e] = __uint_as_float(0x4B000000u | (w[e] & 0xffffu)) - 8388608.f;
-            v[2 * e + 1] = __uint_as_float(0x4B000000u | (w[e] >> 16)) - 8388608.f;
-        }
-    } else if (L.vec) {
-        const float4 *src = reinterpret_cast<const float4 *>(static_cast<const float *>(L.in) + off + j0);
-        const float4 a = __ldg(src), b = (j0 + 4 < L.W) ? __ldg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
-        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
-    } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = (j0 + e < L.W) ? load_raw(L, off, j0 + e) : 0.f;
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-        if (j0 + e >= L.W) v[e] = 0.f;
+    for (int e = 0; e < 8; ++e) v[e] = (j0 + e < L.W) ? load_raw(L, off, j0 + e) : 0.f;
 }
 
 // 16-byte asynchronous copy global -> shared (L2 only), and its groups.
@@ -183,10 +166,14 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+template <int BYTES> __device__ __forceinline__ void cp_async(uint32_t dst, const void *src)  // 4 or 8 bytes
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_prior() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-// Raw-run staging of the producers (rows 16-byte aligned): per stage, item and
+// Raw-run staging of the producers (rows 4-byte aligned or better): per stage, item and
 // 16-byte half, one 16-byte slot per producer thread (consecutive threads on
 // consecutive slots), two stages.
 constexpr int kToepRawBytes = 2 * 4 * 2 * kToepProdWarps * 32 * 16;
@@ -201,7 +188,11 @@ __device__ __forceinline__ long long frame_row(const ToepParams &P, long long gr
     return bf * H + r;
 }
 
-template <int MODE>
+// PLAIN: rows 16-byte aligned, no dark or flat map (with the general code the producers spill more and 300 frames of
+// 256^2 uint16 take 118 us instead of 108).  The general form copies rows in 8- or 4-byte units where they are only
+// aligned to those, instead of loading sample by sample, and reads a run's maps together: 300 frames of W^2 uint16
+// into FP16, W = 500 648 -> 457 us, 300 260 -> 199; with maps W = 256 234 -> 194, 384 546 -> 450, 512 931 -> 772.
+template <int MODE, bool PLAIN>
 __global__ void __launch_bounds__(kToepThreads, 1) filter_toeplitz_kernel(const __grid_constant__ ToepParams P)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -254,15 +245,24 @@ __global__ void __launch_bounds__(kToepThreads, 1) filter_toeplitz_kernel(const 
     const uint32_t tmem = *s_tmem;
     const float sigma = P.q_scale ? *P.q_scale : 1.f;
 
-    if (warp < kToepProdWarps && P.L.vec) {
-        // ---------------------------------------------------------------- producers (aligned rows)
+    auto preprocess = [&](int r, int j0, float (&v)[8]) {
+        const float rt = weight_row_term(P.L, r);
+        if (!PLAIN && has_maps(P.L)) {
+            pre8_maps(P.L, r, j0, rt, v);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = (j0 + e < W) ? pre_from_raw(P.L, r, j0 + e, v[e], rt) : 0.f;
+        }
+    };
+    if (warp < kToepProdWarps && (PLAIN || P.L.gran)) {
+        // ---------------------------------------------------------------- producers (rows aligned to 4 bytes or more)
         // As below, with each thread's runs of a group of four items copied into shared memory
         // asynchronously one group ahead (cp.async), so that the global-load latency overlaps the
         // conversion of the previous group.  Units u of a tile: chunk u / ngroups, group u % ngroups.
         const int pt = tid;
         constexpr int kMaxItems = 8;
         const int nitems = R / 32, g8 = pt & 7, ngroups = (nitems + 3) / 4, nunits = nk * ngroups;
-        const bool f32in = P.L.input_type != TK_INPUT_U16;
+        const bool f32in = P.L.input_type != TK_INPUT_U16, whole = PLAIN || P.L.gran == 16;
         const int esz = f32in ? 4 : 2;
         auto slot16 = [&](int st, int m, int h) -> unsigned char * {
             return raw + ((size_t)(((st * 4 + m) * 2 + h) * (kToepProdWarps * 32) + pt) << 4);
@@ -287,6 +287,25 @@ __global__ void __launch_bounds__(kToepThreads, 1) filter_toeplitz_kernel(const 
                 const int kc = u / ngroups, g = u - kc * ngroups, st = u & 1;
                 const int j0 = P.Wk - 8 - (kc * 64 + g8 * 8);
                 if (j0 >= W) return;  // the run lies past the row: zeros, nothing to copy
+                if (!whole) {  // rows aligned to 8 or 4 bytes only: copies of that size
+                    const int gran = P.L.gran, bytes = min(8, W - j0) * esz;  // whole units: rows end on them
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const int r = g ? rq[4 + m] : rq[m];
+                        if (r < 0) continue;
+                        const char *src = static_cast<const char *>(P.L.in) + ((g ? off[4 + m] : off[m]) + j0) * esz;
+#pragma unroll
+                        for (int k = 0; k < 32; k += 4) {
+                            if (k >= bytes) break;
+                            const uint32_t dst = smem_u32(slot16(st, m, k >> 4)) + (uint32_t)(k & 15);
+                            if (gran == 4)
+                                cp_async<4>(dst, src + k);
+                            else if (k % 8 == 0)
+                                cp_async<8>(dst, src + k);
+                        }
+                    }
+                    return;
+                }
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
                     const int r = g ? rq[4 + m] : rq[m];
@@ -336,9 +355,7 @@ __global__ void __launch_bounds__(kToepThreads, 1) filter_toeplitz_kernel(const 
                                 v[6] = __uint_as_float(b2.z), v[7] = __uint_as_float(b2.w);
                             }
                         }
-                        const float rt = weight_row_term(P.L, r);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] = (j0 + e < W) ? pre_from_raw(P.L, r, j0 + e, v[e], rt) : 0.f;
+                        preprocess(r, j0, v);
                     }
                     // core row: element cc holds column j0 + 7 - cc (the reversed K order)
                     uint4 h, l;
@@ -406,12 +423,7 @@ __global__ void __launch_bounds__(kToepThreads, 1) filter_toeplitz_kernel(const 
                     for (int m = 0; m < 4; ++m) {
                         if (m0 + m >= nitems) break;
                         const int r = rq[m0 + m];
-                        if (r >= 0 && j0 < W) {
-                            const float rt = weight_row_term(P.L, r);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e)
-                                if (j0 + e < W) v[m][e] = pre_from_raw(P.L, r, j0 + e, v[m][e], rt);
-                        }
+                        if (r >= 0 && j0 < W) preprocess(r, j0, v[m]);
                         // core row: element cc holds column j0 + 7 - cc (the reversed K order)
                         uint4 h, l;
                         split_bf16x2(v[m][7], v[m][6], h.x, l.x);
@@ -672,14 +684,19 @@ int launch_filter_toeplitz(const LoadParams &L, const float *Hf, int p, void *d_
         std::memcpy(P.khl, it->second.data(), it->second.size() * sizeof(uint32_t));
     }
     const size_t smem = 1024 + (size_t)P.ncores * 256 + (size_t)P.slots * 2 * P.R * 128 +
-                        (size_t)2 * 33 * kToepPitch * 4 + 22 * 8 + 128 + (L.vec ? kToepRawBytes : 0);
+                        (size_t)2 * 33 * kToepPitch * 4 + 22 * 8 + 128 + (L.gran ? kToepRawBytes : 0);
     TK_CHECK(smem <= 227 * 1024, TK_ERR_UNSUPPORTED, "filter: Toeplitz form needs %zu B of shared memory", smem);
+    const bool plain = L.gran == 16 && !has_maps(L);
     const void *fn = nullptr;
     switch (precision) {
-    case TK_F32: fn = reinterpret_cast<const void *>(&filter_toeplitz_kernel<TK_F32>); break;
-    case TK_F16: fn = reinterpret_cast<const void *>(&filter_toeplitz_kernel<TK_F16>); break;
-    case TK_BF16: fn = reinterpret_cast<const void *>(&filter_toeplitz_kernel<TK_BF16>); break;
-    default: fn = reinterpret_cast<const void *>(&filter_toeplitz_kernel<TK_F32_COEF>); break;
+#define TK_TOEP(MODE)                                                                       \
+    fn = plain ? reinterpret_cast<const void *>(&filter_toeplitz_kernel<MODE, true>)         \
+               : reinterpret_cast<const void *>(&filter_toeplitz_kernel<MODE, false>)
+    case TK_F32: TK_TOEP(TK_F32); break;
+    case TK_F16: TK_TOEP(TK_F16); break;
+    case TK_BF16: TK_TOEP(TK_BF16); break;
+    default: TK_TOEP(TK_F32_COEF); break;
+#undef TK_TOEP
     }
     TK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int dev = 0, sms = 0;
