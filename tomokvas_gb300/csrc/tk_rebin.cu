@@ -46,9 +46,43 @@ struct RebinShifts {
 // the loads of kRebinBatch angles are issued together.  Bound by HBM: 256 rows
 // of 720 x 520 samples into 720 x 997 take 1930 us with one thread per output
 // sample in flat order (64-bit divisions, a divergent parameter read and two
-// loads per sample) and 372 us in this form (1.12 GB moved).
+// loads per sample) and 213 us in this form (1.12 GB moved).
+// Where a batch's angles neither wrap nor change conjugate (all but a few
+// batches) its samples lie one row apart and need no index arithmetic, which
+// otherwise bounds the kernel (ALU pipe 78 %, 61 instructions per sample).
 constexpr int kRebinThreads = 128;
 constexpr int kRebinBatch = 8;
+
+// One such batch: upper samples at rows hi, hi + 1, ... of img, lower samples one row above them, the lower one's
+// weight q (0: the upper sample alone).  `held` is the row whose sample `last` is.
+__device__ __forceinline__ void rebin_rows(const float *__restrict__ img, int W, int hi, float q, int &held, float &last,
+                                           float *&dst, long long ostep)
+{
+    const float *p = img + (long long)hi * W;
+    float A[kRebinBatch];
+#pragma unroll
+    for (int j = 0; j < kRebinBatch; ++j) {
+        A[j] = __ldg(p);
+        p += W;
+    }
+    if (q != 0.f) {
+        if (held != hi - 1) last = __ldg(img + (long long)(hi - 1) * W);
+#pragma unroll
+        for (int j = 0; j < kRebinBatch; ++j) {
+            *dst = A[j] + (last - A[j]) * q;
+            last = A[j];
+            dst += ostep;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < kRebinBatch; ++j) {
+            *dst = A[j];
+            dst += ostep;
+        }
+        last = A[kRebinBatch - 1];
+    }
+    held = hi + kRebinBatch - 1;
+}
 
 // Half2FullFan (rsq_load.cpp:327-380): output row width Wc = 2W - 1 - 2am.
 // Columns c >= W-1-am copy the measured half (from the axis column on);
@@ -78,6 +112,14 @@ __global__ void __launch_bounds__(kRebinThreads)
         int held = -1;  // the angle whose sample `last` is
         float last = 0.f;
         for (int f = f0; f < f1; f += kRebinBatch) {
+            {  // whole batch copied, or from the first, or from the other conjugate, inside [1, N - 1]
+                const int a = f - k0, b = f - k1, n1 = N - kRebinBatch;
+                const bool first = a >= 1 && a <= n1, other = (a + kRebinBatch <= 0 || a > N) && b >= 1 && b <= n1;
+                if (f + kRebinBatch <= f1 && (copy || first || other)) {
+                    rebin_rows(img, W, copy ? f : first ? a : b, copy ? 0.f : first ? fr0 : fr1, held, last, dst, ostep);
+                    continue;
+                }
+            }
             int hi[kRebinBatch], lo[kRebinBatch];
             float fr[kRebinBatch], A[kRebinBatch];
 #pragma unroll
@@ -142,6 +184,15 @@ __global__ void __launch_bounds__(kRebinThreads)
         int held = -1;  // the angle whose sample `last` is
         float last = 0.f;
         for (int f = f0; f < f1; f += kRebinBatch) {
+            {
+                int fb = f + k;
+                if (fb < 0) fb += N;
+                if (fr > 0.f ? fb >= N - 1 : fb > N - 1) fb -= N;
+                if (f + kRebinBatch <= f1 && fb >= 0 && fb + kRebinBatch <= N - 1) {
+                    rebin_rows(img, W, fr != 0.f ? fb + 1 : fb, fr != 0.f ? 1.f - fr : 0.f, held, last, dst, Wc);
+                    continue;
+                }
+            }
             int up[kRebinBatch], dn[kRebinBatch];
             float A[kRebinBatch];
 #pragma unroll
