@@ -1217,9 +1217,9 @@ __global__ void __launch_bounds__(TX *TY, 2)
 // pipe (58 %).  The scatter with slice lanes and two-word integer atomics
 // (fp_scatter_col_kernel) took 62 instructions and 16.7 shared wavefronts, eight
 // atomics of two wavefronts each, for the same (here 12.2).  Measured, that form
-// -> this one: 512^3 at scale 1.5 into 360 x 768^2 94.9 -> 73.8 ms; 256^2 x 224
-// at scale 1.2 into 240 x 320 x 272 7.71 -> 5.56 ms; 256^3 at scale 1 into
-// 180 x 256^2 5.63 -> 4.08 ms; 48^2 x 40 into 60 x 64^2 0.331 -> 0.133 ms.
+// -> this one: 512^3 at scale 1.5 into 360 x 768^2 94.9 -> 72.5 ms; 256^2 x 224
+// at scale 1.2 into 240 x 320 x 272 7.71 -> 5.47 ms; 256^3 at scale 1 into
+// 180 x 256^2 5.63 -> 4.05 ms; 48^2 x 40 into 60 x 64^2 0.331 -> 0.132 ms.
 struct FpRows {
     int TZ;       // slices of a chunk
     int GP;       // voxels of a column in shared memory, padding included (odd)
@@ -1373,6 +1373,7 @@ __global__ void __launch_bounds__(32 * kFpWarps, 2)
             *reinterpret_cast<float4 *>(rowa + c) = make_float4(0.f, 0.f, 0.f, 0.f);
             *reinterpret_cast<float4 *>(rowb + c) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
+        asm volatile("" ::: "memory");  // the walk's accesses to the box are in assembly
         // the table entry of column j: (U, A, B, voxel address), then its weights for the even and the odd one of
         // the detector columns c, c + 1 (U^2 (1 - fu) for c, U^2 fu for c + 1) and their byte offsets in a row.
         // The columns reached are stored one after another from slot n on.
@@ -1406,13 +1407,28 @@ __global__ void __launch_bounds__(32 * kFpWarps, 2)
         // sums of the two rows over the columns whose even cell is pe, odd cell po (byte offsets)
         float ea = 0.f, eb = 0.f, oa = 0.f, ob = 0.f;
         uint32_t pe = 0u, po = 4u;
-        auto put = [&](uint32_t cell, float va, float vb) {
-            const uint32_t aa = rowa_s + (cell ^ (4u * sw)), ab = aa + row_gap;
-            float qa, qb;
-            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(qa) : "r"(aa));
-            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(qb) : "r"(ab));
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(aa), "f"(qa + va) : "memory");
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(ab), "f"(qb + vb) : "memory");
+        // Moves on from cell `from` to `to`: where they differ, the two rows' sums go to the box.  Both are the same for
+        // the whole warp, which bra.uni says (a branch the compiler cannot prove uniform costs two more
+        // instructions to join again).
+        const uint32_t sw4 = 4u * sw;
+        auto move = [&](uint32_t from, uint32_t to, float &va, float &vb) {
+            asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 a, b;\n\t.reg .f32 qa, qb;\n\t"
+                         "setp.eq.u32 p, %2, %3;\n\t"
+                         "@p bra.uni SAME;\n\t"
+                         "xor.b32 a, %2, %4;\n\t"
+                         "add.u32 a, a, %5;\n\t"
+                         "add.u32 b, a, %6;\n\t"
+                         "ld.shared.f32 qa, [a];\n\t"
+                         "ld.shared.f32 qb, [b];\n\t"
+                         "add.rn.f32 qa, qa, %0;\n\t"
+                         "add.rn.f32 qb, qb, %1;\n\t"
+                         "st.shared.f32 [a], qa;\n\t"
+                         "st.shared.f32 [b], qb;\n\t"
+                         "mov.f32 %0, 0f00000000;\n\t"
+                         "mov.f32 %1, 0f00000000;\n\t"
+                         "SAME:\n\t}"
+                         : "+f"(va), "+f"(vb)
+                         : "r"(from), "r"(to), "r"(sw4), "r"(rowa_s), "r"(row_gap));
         };
         auto walk = [&](auto mask_tag) {
             constexpr bool MASK = decltype(mask_tag)::value;
@@ -1466,16 +1482,10 @@ __global__ void __launch_bounds__(32 * kFpWarps, 2)
             };
             auto add = [&](float ha, float hb, const float4 &e) {
                 const uint32_t ce = __float_as_uint(e.z), co = __float_as_uint(e.w);
-                if (ce != pe) {  // the same for the whole warp
-                    put(pe, ea, eb);
-                    ea = eb = 0.f;
-                    pe = ce;
-                }
-                if (co != po) {
-                    put(po, oa, ob);
-                    oa = ob = 0.f;
-                    po = co;
-                }
+                move(pe, ce, ea, eb);
+                move(po, co, oa, ob);
+                pe = ce;
+                po = co;
                 ea = fmaf(ha, e.x, ea);
                 eb = fmaf(hb, e.x, eb);
                 oa = fmaf(ha, e.y, oa);
@@ -1513,8 +1523,9 @@ __global__ void __launch_bounds__(32 * kFpWarps, 2)
             else
                 walk(std::false_type{});
         }
-        put(pe, ea, eb);
-        put(po, oa, ob);
+        move(pe, 0xffffffffu, ea, eb);
+        move(po, 0xffffffffu, oa, ob);
+        asm volatile("" ::: "memory");  // the box is read as C++ objects from here on
 
         // (4) undo the rows' column order in place, then reduce the box into the gradient
         auto unswizzle = [&](float *row) {
