@@ -301,11 +301,9 @@ __global__ void __launch_bounds__(TX *TY, MINB)
         }
         __syncthreads();  // every thread is done with the step's stages
         if (s_abort) break;
-        if (tid == 0) {
-#pragma unroll
-            for (int i = 0; i < NB; ++i) {
-                const int k = b + i + STAGES;
-                if (k >= P.N) break;
+        {  // warp i refills stage i of the step: one warp doing all would reach the next barrier late
+            const int i = tid >> 5, k = b + i + STAGES;
+            if ((tid & 31) == 0 && i < NB && k < P.N) {
                 mbar_arrive_expect_tx(&full[s0 + i], stage_bytes);
                 tma_load_3d(stages + (size_t)(s0 + i) * P.stage_elems, &tmap, boxo[k].x, boxo[k].y, k, &full[s0 + i]);
             }
