@@ -18,7 +18,7 @@ def test_thin_tiles_same_bits(cuda, X, Y, nz, N, flips):
 
     L = _lib.load()
     names = [L.tk_bp_variant_name(i).decode() for i in range(L.tk_bp_variant_count())]
-    idx = [i for i, n in enumerate(names) if n.startswith("direct_x2<f32,16,16,")]
+    idx = [i for i, n in enumerate(names) if n.startswith("direct_x2<f32,")]
     assert sorted(int(names[i].split(",")[3]) for i in idx) == [4, 8, 32]
     g = FDKGeometry(W=60, N=N, H=37, cX=29.7, cZ=18.2, dfi=float(np.float32(2 * math.pi / N)), D=380.0, tau=0.02, X=X,
                     Y=Y, Z=nz, cx=(X - 1) / 2 + 1.5, cy=(Y - 1) / 2, rot=0.3, scale=1.1, dirx=flips & 1,

@@ -1623,13 +1623,13 @@ struct BPVariant {
 // the quarter-turn kernel with 16 x 8 tiles, else walk 4.  The half-math
 // walks (FP16 interpolation arithmetic) are selectable only.
 static const BPVariant kVariants[] = {
-    TK_BP_DIRECT_PK(16, 16, 32, 4, 2, 2, false),
+    TK_BP_DIRECT_PK(16, 8, 32, 4, 4, 2, false),
     TK_BP_QUADF(TK_F16, "f16", 6144, 2, true, 8),
-    TK_BP_CIMG_F(TK_F16, "f16", 16, 16, 64, 3, 2),
+    TK_BP_CIMG_F(TK_F16, "f16", 16, 8, 64, 2, 4),
     TK_BP_QUADF(TK_BF16, "bf16", 6144, 2, true, 8),
-    TK_BP_CIMG_F(TK_BF16, "bf16", 16, 16, 64, 3, 2),
+    TK_BP_CIMG_F(TK_BF16, "bf16", 16, 8, 64, 2, 4),
     TK_BP_CIMG_PK(TK_F32_COEF, "f32c", 16, 16, 64, 2, 2),
-    TK_BP_DIRECT(16, 16, 32, 4),
+    TK_BP_DIRECT(16, 8, 32, 4),
     TK_BP_QUADF(TK_F16, "f16", 8192, 2, true, 16),   // 16 x 16 tiles when a 16 x 8 tile's footprint exceeds 6 KB
     TK_BP_QUADF(TK_F16, "f16", 13824, 2, true, 16),  // footprints of up to 13.5 KB (scales near 1.5)
     TK_BP_QUADF(TK_BF16, "bf16", 8192, 2, true, 16),
@@ -1655,10 +1655,9 @@ static const BPVariant kVariants[] = {
     TK_BP_CIMG(TK_F32_COEF, "f32c", 16, 16, 32, 3, 2),
     TK_BP_CIMG(TK_F32_COEF, "f32c", 16, 16, 32, 2, 3),
     // few slices per tile for small FP32 volumes (z_split)
-    TK_BP_DIRECT_PK(16, 16, 8, 12, 4, 4, true),
-    TK_BP_DIRECT_PK(16, 16, 4, 8, 4, 4, true),
-    // two-stage twins of the 16-bit general walks, taken where three staged boxes would leave
-    // room for one CTA per SM only (two_stage_twin)
+    TK_BP_DIRECT_PK(16, 8, 8, 8, 8, 4, true),
+    TK_BP_DIRECT_PK(16, 8, 4, 8, 8, 4, true),
+    // 16 x 16 tiles of the 16-bit general walks for large footprints (wide_twin)
     TK_BP_CIMG_F(TK_F16, "f16", 16, 16, 64, 2, 2),
     TK_BP_CIMG_F(TK_BF16, "bf16", 16, 16, 64, 2, 2),
 };
@@ -1676,31 +1675,29 @@ static const BPVariant *pick_variant(int precision)
     return nullptr;
 }
 
-// The two-stage variant with v's walk, storage and tile shape (the same
-// arithmetic, so the same bits), or null.
-static const BPVariant *two_stage_twin(const BPVariant *v)
+// The 16 x 16 variant with v's walk, storage and slices per tile (the same arithmetic, so the same bits), or null.
+static const BPVariant *wide_twin(const BPVariant *v)
 {
     const char *lt = std::strchr(v->name, '<');
     const size_t np = lt ? (size_t)(lt - v->name) : std::strlen(v->name);
     for (const auto &c : kVariants)
-        if (&c != v && c.precision == v->precision && c.coef == v->coef && !c.qcap && c.STAGES == 2 &&
-            c.TX == v->TX && c.TY == v->TY && c.TZ == v->TZ && std::strncmp(c.name, v->name, np) == 0 &&
-            c.name[np] == '<')
+        if (&c != v && c.precision == v->precision && c.coef == v->coef && !c.qcap && c.TX == 16 && c.TY == 16 &&
+            c.TZ == v->TZ && std::strncmp(c.name, v->name, np) == 0 && c.name[np] == '<')
             return &c;
     return nullptr;
 }
 
 // The FP32 variant for `columns` tiles per slice layer and nz slices: the default (32 slices per tile), or the same
 // walk with 8 or 4, where tiles of 32 would leave SMs idle or walk slices past the end.  Estimates of the time per 96
-// projections in us from x CTAs per SM, fitted to cubes of 32 to 256 and to slabs: 32 slices max(108, 55 + 65 x),
-// 8 slices 40 + 19.5 x, 4 slices 25 + 14.2 x (a step's geometry, wait and barrier cost about three slices).
-// Measured, 32 / 8 / 4 slices: 64^2 x 48 109 / 54 / 53 us, 80^2 x 64 109 / 68 / 63, 96^3 132 / 94 / 123, 128^3
-// 191 / 181 / 223, 160^3 277 / 299 / 390, 512^2 x 16 430 / 288 / 373.
+// projections in us from x CTAs per SM, fitted to cubes of 32 to 256 and to slabs: 32 slices max(80, 75 + 27.5 x),
+// 8 slices 42 + 9.4 x, 4 slices 30 + 6.7 x (a step's geometry, wait and barrier cost about three slices).
+// Measured, 32 / 8 / 4 slices: 64^2 x 48 79 / 53 / 47 us, 96^3 127 / 94 / 107, 128^3 169 / 170 / 211, 160^3
+// 252 / 286 / 376, 512^2 x 16 421 / 275 / 361.
 static const BPVariant *z_split(const BPVariant *v, long long columns, int nz, int sms)
 {
     auto cost = [&](int TZ) {
         const double x = (double)(columns * ((nz + TZ - 1) / TZ)) / sms;
-        return TZ == 32 ? std::max(108.0, 55.0 + 65.0 * x) : TZ == 8 ? 40.0 + 19.5 * x : 25.0 + 14.2 * x;
+        return TZ == 32 ? std::max(80.0, 75.0 + 27.5 * x) : TZ == 8 ? 42.0 + 9.4 * x : 30.0 + 6.7 * x;
     };
     const BPVariant *best = v;
     for (const auto &c : kVariants)
@@ -1828,16 +1825,33 @@ static int launch_bp_impl(const tk_geometry &g, const void *d_q, int precision, 
     const int align = v->coef ? (ES >= 16 ? 1 : 16 / ES) : 4;
     int BW, BH;
     if (int rc = bp_box_dims(g, nz, zoff, v->TX, v->TY, v->TZ, v->coef, align, &BW, &BH)) return rc;
-    // A 16-bit general walk whose three staged boxes would fit one CTA per SM only (large
-    // footprints: scale near 1.5 at high magnification) takes its two-stage twin, which keeps two.
-    if (v->coef && !quad && v->STAGES == 3 && g_variant_override < 0 && precision != TK_F32_COEF) {
-        int dev = 0, per_sm = 0;
-        TK_CUDA(cudaGetDevice(&dev));
-        TK_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-        const size_t box = (size_t)((BW * BH + 15) / 16 * 16) * ES;
-        const size_t fixed = (size_t)std::min(g.N, kMaxParamProj) * sizeof(int2) + 3 * sizeof(uint64_t) + 16;
-        if (3 * box + fixed + 1024 > (size_t)per_sm / 2)  // 1 KB reserved per CTA
-            if (const BPVariant *t = two_stage_twin(v)) v = t;
+    const int nb_max = std::min(g.N, kMaxParamProj);
+    if (!quad && g_variant_override < 0 && precision != TK_F32_COEF) {
+        // The default tiles are 16 x 8 columns, four CTAs of 128 threads per SM (their barriers join four warps, and
+        // the last CTAs are half as long): 256^3 FP32 samples from 96 projections 879 -> 819 us, 512^3 6295 -> 6017;
+        // 333^2 x 201 BF16 from 301 at scale 1.1 3239 -> 3151, 500^3 FP16 from 200 13506 -> 13010 (16 x 16, two CTAs of
+        // 256).  A 16-bit walk whose boxes do not leave room for four takes 16 x 16 tiles where those keep more warps
+        // on an SM (512^3 at scale 1.45: 11325 us against 11479).  What 16 x 16 tiles cannot do is refused.
+        int wBW, wBH;
+        if (int rc = bp_box_dims(g, nz, zoff, 16, 16, v->coef ? 64 : 32, v->coef, align, &wBW, &wBH)) return rc;
+        TK_CHECK(!v->coef || wBW * ES / 4 <= 256, TK_ERR_UNSUPPORTED, "tile footprint of %d entries too wide", wBW);
+        const size_t fixed = (size_t)nb_max * sizeof(int2) + 4 * sizeof(uint64_t) + 16;
+        const size_t wide = v->coef ? 2 * (size_t)((wBW * wBH + 15) / 16 * 16) * ES + fixed
+                                    : 4 * (size_t)((wBW * wBH + 63) / 64 * 64) * ES + fixed;
+        TK_CHECK(wide <= 227 * 1024, TK_ERR_UNSUPPORTED, "backproject: %zu B of shared memory needed", wide);
+        if (v->coef) {
+            int dev = 0, per_sm = 0;
+            TK_CUDA(cudaGetDevice(&dev));
+            TK_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+            const size_t own = 2 * (size_t)((BW * BH + 15) / 16 * 16) * ES + fixed;
+            const size_t warps = 4 * std::min<size_t>(4, per_sm / (own + 1024));  // 1 KB reserved per CTA
+            const BPVariant *w = wide_twin(v);
+            if (w && 8 * std::min<size_t>(2, per_sm / (wide + 1024)) > warps) {
+                v = w;
+                BW = wBW;
+                BH = wBH;
+            }
+        }
     }
     BH = std::max(1, BH - g_diag_box_shrink);  // 0 unless a self-check test shrinks the staged box
     TK_CHECK(!v->coef || BW * ES / 4 <= 256, TK_ERR_UNSUPPORTED, "tile footprint of %d entries too wide", BW);
