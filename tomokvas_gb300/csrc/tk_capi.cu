@@ -1096,6 +1096,15 @@ extern "C" int tk_fdk_calculate_reconstruction(tk_fdk *h, tk_block_sink sink, vo
         TK_CUDA(cudaEventRecord(h->ev_filt, h->stream));
         TK_CUDA(cudaStreamWaitEvent(h->aux_stream, h->ev_filt, 0));  // the filter, and earlier work on the stream
     }
+    // However this call ends (a sink that returns NULL or throws included), no block is left running on the second
+    // stream: what follows on the handle is ordered after the first one only.
+    struct AuxDone {
+        tk_fdk *h;
+        ~AuxDone()
+        {
+            if (h->aux_stream) cudaStreamSynchronize(h->aux_stream);
+        }
+    } aux_done{h};
     auto launch_block = [&](int n) -> int {
         const int k = n & 1;
         cudaStream_t st = k ? h->aux_stream : h->stream;
