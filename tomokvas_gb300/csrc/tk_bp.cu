@@ -151,7 +151,8 @@ __device__ __forceinline__ void direct_update(uint32_t sbase, uint32_t row_bytes
     if constexpr (PACKED && (TZ % 2 == 0)) {
 #pragma unroll
         for (int z = 0; z < TZ; z += 2) {
-            const float va = slice_v(aZ[z], U, cZ), vb = slice_v(aZ[z + 1], U, cZ);
+            float va, vb;
+            slice_v_x2(aZ[z], aZ[z + 1], U, cZ, va, vb);
             float fla, flb, fva, fvb;
             floor_frac_x2(va, vb, fla, flb, fva, fvb);
             const uint32_t oa = (uint32_t)__float_as_int(fla) * row_bytes + sbase;
@@ -1211,10 +1212,10 @@ __global__ void __launch_bounds__(TX *TY, 2)
 // kernel's voxel by voxel; a slice estimate that rounds to a neighbour loses
 // only weights of a few ulps, because the hat is continuous.
 //
-// Bound by issue (66 %, 56 warp-instructions per 32 updates) beside the shared
-// pipe (58 %).  The scatter with slice lanes and two-word integer atomics
-// (fp_scatter_col_kernel) took 62 instructions and 16.7 shared wavefronts, eight
-// atomics of two wavefronts each, for the same (here 12.2).  Measured, that form
+// Bound by issue (71 %, 43 warp-instructions per 32 voxels and projection)
+// beside the shared pipe (63 %, 9.6 wavefronts).  The scatter with slice lanes
+// and two-word integer atomics (fp_scatter_col_kernel) took 62 instructions and
+// 16.8 shared wavefronts, eight atomics among them.  Measured, that form
 // -> this one: 512^3 at scale 1.5 into 360 x 768^2 94.9 -> 72.5 ms; 256^2 x 224
 // at scale 1.2 into 240 x 320 x 272 7.71 -> 5.47 ms; 256^3 at scale 1 into
 // 180 x 256^2 5.63 -> 4.05 ms; 48^2 x 40 into 60 x 64^2 0.331 -> 0.132 ms.

@@ -168,6 +168,19 @@ __device__ __forceinline__ void floor_frac_x2(float va, float vb, float &fla, fl
         : "=f"(fla), "=f"(flb), "=f"(fva), "=f"(fvb)
         : "f"(va), "f"(vb), "f"(kMagic));
 }
+// slice_v of two slices as one fma.rn.f32x2 (the same rounding each).  One issue slot less per pair of the direct
+// FP32 walk: 256^3 from 180 x 256^2 1583 -> 1557 us per reconstruction.
+__device__ __forceinline__ void slice_v_x2(float aZa, float aZb, float U, float cZ, float &va, float &vb)
+{
+    asm("{\n\t.reg .b64 A, D, C;\n\t"
+        "mov.b64 A, {%2, %3};\n\t"
+        "mov.b64 D, {%4, %4};\n\t"
+        "mov.b64 C, {%5, %5};\n\t"
+        "fma.rn.f32x2 A, A, D, C;\n\t"
+        "mov.b64 {%0, %1}, A;\n\t}"
+        : "=f"(va), "=f"(vb)
+        : "f"(aZa), "f"(aZb), "f"(U), "f"(cZ));
+}
 // (va, vb) += (d, d) as one add.rn.f32x2.
 __device__ __forceinline__ void add_pair(float &va, float &vb, float d)
 {
