@@ -68,8 +68,8 @@ def half_math_variant():
 # (one ncu pass on the 64-slice slab case, so the full-size launch is captured in one pass, nothing saved or
 # restored).  source_sha1 is the sha1 of tk_bp.cu + tk_bp_core.cuh at capture: a later source reports the
 # traffic as stale (null) instead of a frozen number.
-BP_TRAFFIC = {"kernel": "bp_quad<f16,16,8,16,2,cap6144,f32i,issue1,geo1>", "bytes_per_launch": 310.51e9 + 4.30e9,
-              "source_sha1": "a79e5ca07db27cf4acb4799b067280a168fc95b7",
+BP_TRAFFIC = {"kernel": "bp_quad<f16,16,8,16,2,cap6144,f32i,issue1,geo1>", "bytes_per_launch": 343.89e9 + 4.30e9,
+              "source_sha1": "65a984c9fcfe4ac49faff433ea4ee105581eb778",
               "capture": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none "
                          "-k regex:bp_quad -c 1 python bench.py --steps 1 --warmup 1 --no-e2e --no-rmse --no-extras"}
 
@@ -917,7 +917,7 @@ def adjoint_summary(steps, warmup, column_lanes=False, descent_p=False, refine_s
             "monotone": bool(np.all(np.diff(ls) < 0)),
             "launches_per_step": (L.tk_kernel_launches() - n0) / refine_steps,
             "checkpoint": "filtered projections q = F W p as FP16 samples (0.42 GB instead of 0.85 GB FP32)",
-            "per_step": "B^T x (scatter forward projector) + residual -alpha (B^T x - q) with the loss + "
+            "per_step": "B^T x (forward projector) + residual -alpha (B^T x - q) with the loss + "
                         "B r accumulated into x (FP32 backprojector)"}
         del rws, ck, x
     res["flags"] = device.device_error_flags()
