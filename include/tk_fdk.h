@@ -292,7 +292,7 @@ int tk_bp_variant_count(void);
 const char *tk_bp_variant_name(int i);
 int tk_bp_variant_precision(int i);
 int tk_bp_select_variant(int i);
-/* Forward projector (the scatter of tk_forward_project / tk_fdk_backward):
+/* Forward projector (tk_forward_project / tk_fdk_backward):
  * 0 (default) lanes on detector rows, gathering the slices that reach them
  * (FP32 sums without atomics in the box); where that does not apply (row steps
  * below 1/2, very large footprints) lanes on 32 consecutive slices of one voxel

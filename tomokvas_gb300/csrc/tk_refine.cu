@@ -8,7 +8,7 @@
 // refinement minimises the data-consistency loss
 //   L(x) = || B^T x - q ||^2
 // over the volume by gradient steps x <- x - alpha B (B^T x - q), with B^T the
-// scatter forward projector that is B's exact transpose (tk_forward_project).
+// forward projector that is B's exact transpose (tk_forward_project).
 // q is the only data a step needs besides x, so it is checkpointed once after
 // the filter: in FP32 samples, or where HBM is short in FP16 samples (half the
 // bytes, the residual formed in FP32).  A step is three launches: B^T x into
