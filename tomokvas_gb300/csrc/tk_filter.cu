@@ -16,6 +16,7 @@
 // conj(FFT(conj(Z) * Hf)).  Results are written once, projection-major, in
 // FP32/FP16/BF16.  No cuFFT, no staging copies, no per-row plans.
 #include "tk_common.cuh"
+#include "tk_fft_shape.h"
 #include "tk_filter_core.cuh"
 #include "tk_internal.h"
 
@@ -29,7 +30,6 @@
 namespace tk {
 
 constexpr int kMaxHf = 4097;  // p/2 + 1 for p <= 8192
-constexpr int kFiltThreads = 256;
 constexpr float kScaleTarget = 16384.f;  // bound of |stored value| for 16-bit storage
 
 // ---------------------------------------------------------------------------
@@ -54,40 +54,6 @@ constexpr float kScaleTarget = 16384.f;  // bound of |stored value| for 16-bit s
 // Buffers are padded by one element per 16 (pidx), which makes every pass's
 // loads and stores conflict-free; twiddles come from per-pass tables laid out
 // [k][r] (one thread reads R-1 consecutive entries).
-
-// Threads per transform (one radix-16 butterfly each); compile-time form.
-__host__ __device__ constexpr int fft_threads_c(int p)
-{
-    return ((p >> 4) > 32 ? (p >> 4) : 32) < kFiltThreads ? ((p >> 4) > 32 ? (p >> 4) : 32) : kFiltThreads;
-}
-
-// Shape of the length-2^LG filter.
-template <int LG> struct Fft {
-    static constexpr int P = 1 << LG, NP = (LG + 3) / 4;              // passes of one transform
-    static constexpr int RL = LG % 4 ? 1 << (LG % 4) : 16;            // radix of the last forward pass
-    static constexpr int R1 = NP > 1 ? 16 : RL, Q1 = P / R1;          // first pass: radix and butterflies
-    static constexpr int TPF = fft_threads_c(P), G = kFiltThreads / TPF;
-    static constexpr int IN = R1 / 2, ITIN = (Q1 + TPF - 1) / TPF;    // samples j + r Q1, r < IN, per butterfly
-    // output columns j + s QC, s < NC, of butterfly j of the last pass
-    static constexpr int NC = NP > 1 ? 8 : 1, QC = NP > 1 ? P / 16 : P / 2, ITC = (QC + TPF - 1) / TPF;
-    // twiddle tables: forward passes m >= 1 (span 16^m), then the inverse's radix-16 passes (span RL 16^m).
-    // RL = 16: the same tables.  LG = 13: the last forward table, w^k for k < p/2, serves the inverse.
-    static constexpr int fwd_off(int m) { return m >= 1 ? (1 << (4 * m)) - 16 : 0; }
-    static constexpr int FWD = NP > 1 ? fwd_off(NP - 1) + (P / RL) * (RL - 1) : 0;
-    static constexpr bool OWN_INV = RL != 16 && LG < 13 && NP > 1;
-    static constexpr int inv_span(int m) { return RL << (4 * m); }    // m = 0 .. NP - 2
-    static constexpr int inv_off(int m)
-    {
-        int o = OWN_INV ? FWD : 0;
-        for (int i = 0; i < m; ++i) o += inv_span(i) * 15;
-        return o;
-    }
-    static constexpr int TW = OWN_INV ? inv_off(NP - 1) : FWD;        // entries of all tables
-    static constexpr int HF = ((P / 2 + 1) + 3) & ~3;                 // spectrum, floats
-    static constexpr int EDGE = (TPF / 32) * (NC + 1);                // first columns of each warp, float2
-    static constexpr size_t group_bytes() { return (size_t)(2 * (P + P / 16) + EDGE) * 8; }
-    static constexpr size_t smem() { return (size_t)TW * 8 + HF * 4 + G * group_bytes(); }
-};
 
 struct FiltParams {
     LoadParams L;
@@ -654,8 +620,7 @@ __global__ void __launch_bounds__(kFiltThreads) filter_coef_kernel(const __grid_
                 for (int s2 = 0; s2 < NC; ++s2) S.edge[(t >> 5) * (NC + 1) + s2] = q[0][s2];
             }
             group_sync<F::TPF>(grp);
-            const bool last = t == F::QC - 1;  // its next column is the first of the next s
-            const float2 *edge = S.edge + (last ? 1 : ((t >> 5) + 1) * (NC + 1));
+            const int next = F::next_edge(t);
             const size_t base = ((size_t)bf * H + ra) * Wc;
 #pragma unroll
             for (int s2 = 0; s2 < NC; ++s2) {
@@ -664,7 +629,7 @@ __global__ void __launch_bounds__(kFiltThreads) filter_coef_kernel(const __grid_
                 float2 n;
                 n.x = __shfl_down_sync(0xffffffffu, v.x, 1);
                 n.y = __shfl_down_sync(0xffffffffu, v.y, 1);
-                if (last || lane == 31) n = c + 1 < W ? edge[s2] : make_float2(0.f, 0.f);
+                if (next >= 0) n = c + 1 < W ? S.edge[next + s2] : make_float2(0.f, 0.f);
                 const float da = n.x - v.x, db = n.y - v.y;
                 if (live && t < F::QC && c < Wc) {
                     if (ra - 1 >= r0)  // the previous row, followed by row ra
