@@ -551,6 +551,10 @@ __global__ void __launch_bounds__(kFiltThreads) filter_fft_kernel(const __grid_c
 // which the last coefficient row needs) and keeps the previous filtered row in
 // registers (each thread holds it at its own columns), so every coefficient
 // row r is formed from filtered rows r and r+1 without another pass over HBM.
+// Rows 2i and 2i + 1 of a frame always share a transform, the next unit's first
+// row and its partner too (the partner is used there only): a transform's
+// rounding depends on both of its rows, and RC on the number of frames in the
+// call, which a frame's entries must not follow.
 // A thread's columns are j + s QC; column c + 1 sits in the next lane, or, for
 // the last lane of a warp, in the next warp's first columns, which pass through
 // shared memory.  Samples outside the detector are 0.
@@ -589,7 +593,7 @@ __global__ void __launch_bounds__(kFiltThreads) filter_coef_kernel(const __grid_
         auto fetch = [&](int kk) {
             const bool lv = valid && kk < npair;
             const int qa = r0 + 2 * kk, qb = qa + 1;
-            const bool hb = lv && qb <= rend;
+            const bool hb = lv && qb < H;
             int rr;
             const long long oa = lv ? in_row_offset(P.L, bf * H + qa, rr) : 0;
             const long long ob = hb ? in_row_offset(P.L, bf * H + qb, rr) : 0;
@@ -603,7 +607,7 @@ __global__ void __launch_bounds__(kFiltThreads) filter_coef_kernel(const __grid_
         for (int k = 0; k < steps; ++k) {
             const bool live = valid && k < npair;
             const int ra = r0 + 2 * k, rb = ra + 1;
-            const bool hasb = live && rb <= rend;
+            const bool hasb = live && rb < H;
             float2 in[1][F::IN], q[1][NC];
             pack_inputs<LG>(P.L, ra, rb, live, hasb, t, raw_a, raw_b, in);
             if (k + 1 < steps) fetch(k + 1);
