@@ -1,6 +1,6 @@
 """Index rules of the FFT filter on the host (tests/cpp/fft_shape_check.cpp over csrc/tk_fft_shape.h), and on the GPU the
-widths at which a group's warp covers fewer than 32 butterflies (pad lengths 128 and 256), where a thread without a
-column once read another group's buffer.
+widths of few butterflies (pad lengths to 256), whose transforms share a warp and where a thread without a column once
+read another group's buffer.
 
 GPU bound: as for the other lengths, the FP32 transform's error is below 2e-6 of the filtered rows' RMS (about log2(p)
 roundings of 2^-24 per value, random rows); dU, dV and dUV are differences of such values, formed in FP32: 4e-6 relative
@@ -28,7 +28,7 @@ def test_edge_reads_stay_in_their_group(tmp_path):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("W", [33, 63, 64, 65, 100, 112, 127, 128])
+@pytest.mark.parametrize("W", [1, 3, 4, 5, 8, 9, 16, 17, 31, 32, 33, 63, 64, 65, 100, 112, 127, 128])
 def test_coefficients_of_narrow_rows(orc, cuda, W):
     import torch
 

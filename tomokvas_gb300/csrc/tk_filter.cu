@@ -226,12 +226,16 @@ template <int R> __device__ __forceinline__ void dft_half(float2 (&v)[R])
     }
 }
 
-// Barrier of the TPF threads of transform group grp (named barrier 1 + grp):
-// the groups of a CTA share only read-only tables, so none waits on another.
+// Barrier of the TPF threads of transform group grp (named barrier 1 + grp, or
+// the warp's own where groups share a warp): the groups of a CTA share only
+// read-only tables, so none waits on another.
 template <int TPF>
 __device__ __forceinline__ void group_sync(int grp)
 {
-    asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(TPF) : "memory");
+    if constexpr (TPF < 32)
+        __syncwarp();
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(TPF) : "memory");
 }
 
 // Loads of butterfly j of a radix-R pass: x[j + r Q] times its twiddles.
@@ -491,14 +495,14 @@ __device__ __forceinline__ void pack_inputs(const LoadParams &L, int r_a, int r_
 }
 
 template <int LG>
-__global__ void __launch_bounds__(kFiltThreads) filter_fft_kernel(const __grid_constant__ FiltParams P)
+__global__ void __launch_bounds__(Fft<LG>::NT, Fft<LG>::MINB) filter_fft_kernel(const __grid_constant__ FiltParams P)
 {
     extern __shared__ __align__(16) float2 fsm[];
     using F = Fft<LG>;
     const int grp = threadIdx.x / F::TPF, t = threadIdx.x - grp * F::TPF;
     const FiltSmem<LG> S(fsm, grp);
     fill_twiddles<LG>(S.tw);
-    for (int k = threadIdx.x; k <= F::P / 2; k += kFiltThreads) S.hf[k] = P.Hf[k];
+    for (int k = threadIdx.x; k <= F::P / 2; k += F::NT) S.hf[k] = P.Hf[k];
     const int W = P.L.W;
     float *out = static_cast<float *>(P.out);
     __syncthreads();
@@ -560,16 +564,16 @@ __global__ void __launch_bounds__(kFiltThreads) filter_fft_kernel(const __grid_c
 // shared memory.  Samples outside the detector are 0.
 
 template <int MODE, int LG>
-__global__ void __launch_bounds__(kFiltThreads) filter_coef_kernel(const __grid_constant__ FiltParams P)
+__global__ void __launch_bounds__(Fft<LG>::NT, Fft<LG>::MINB) filter_coef_kernel(const __grid_constant__ FiltParams P)
 {
     extern __shared__ __align__(16) float2 fsm[];
     using F = Fft<LG>;
     static_assert(F::ITC == 1 && F::ITIN == 1, "one butterfly per thread (p <= 4096)");
     constexpr int NC = F::NC;
-    const int grp = threadIdx.x / F::TPF, t = threadIdx.x - grp * F::TPF, lane = threadIdx.x & 31;
+    const int grp = threadIdx.x / F::TPF, t = threadIdx.x - grp * F::TPF;
     const FiltSmem<LG> S(fsm, grp);
     fill_twiddles<LG>(S.tw);
-    for (int k = threadIdx.x; k <= F::P / 2; k += kFiltThreads) S.hf[k] = P.Hf[k];
+    for (int k = threadIdx.x; k <= F::P / 2; k += F::NT) S.hf[k] = P.Hf[k];
     const float sigma = P.q_scale ? *P.q_scale : 1.f;
     const int W = P.L.W, H = P.L.H, RC = P.rc;
     const int Wc = MODE == TK_F32_COEF ? W : ((W + 1) & ~1);
@@ -619,7 +623,7 @@ __global__ void __launch_bounds__(kFiltThreads) filter_coef_kernel(const __grid_
                 q[0][s2] = in_row ? make_float2(q[0][s2].x * sigma, hasb ? -q[0][s2].y * sigma : 0.f)
                                   : make_float2(0.f, 0.f);
             }
-            if (lane == 0) {
+            if (t % 32 == 0) {
 #pragma unroll
                 for (int s2 = 0; s2 < NC; ++s2) S.edge[(t >> 5) * (NC + 1) + s2] = q[0][s2];
             }
@@ -789,13 +793,14 @@ static const Spectrum &spectrum(int W, float tau, int window, int p)
 struct FiltKernel {
     const void *fn = nullptr;
     size_t smem = 0;
-    int groups = 1;
+    int groups = 1, threads = 0;
 };
 template <int LG> static FiltKernel filter_kernel_lg(int precision)
 {
     FiltKernel k;
     k.smem = Fft<LG>::smem();
     k.groups = Fft<LG>::G;
+    k.threads = Fft<LG>::NT;
     switch (precision) {
     case TK_F32: k.fn = reinterpret_cast<const void *>(&filter_fft_kernel<LG>); break;
     case TK_F16: if constexpr (LG <= 12) k.fn = reinterpret_cast<const void *>(&filter_coef_kernel<TK_F16, LG>); break;
@@ -858,7 +863,7 @@ static int launch_filter_typed(FiltParams &P, int p, cudaStream_t stream, int pr
     int dev = 0, sms = 0, per_sm = 0;
     TK_CUDA(cudaGetDevice(&dev));
     TK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    TK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kFiltThreads, smem));
+    TK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, k.threads, smem));
     if (per_sm < 1) per_sm = 1;
     if (is_coef(precision)) {
         P.rc = rows_per_unit(P.L.N, P.L.H, (long long)sms * per_sm * G);
@@ -869,7 +874,7 @@ static int launch_filter_typed(FiltParams &P, int p, cudaStream_t stream, int pr
     const long long groups = (work + G - 1) / G;
     const long long grid = std::min<long long>(groups, (long long)sms * per_sm);
     void *args[] = {&P};
-    TK_CUDA(cudaLaunchKernel(fn, dim3((unsigned)std::max<long long>(grid, 1)), dim3(kFiltThreads), args, smem,
+    TK_CUDA(cudaLaunchKernel(fn, dim3((unsigned)std::max<long long>(grid, 1)), dim3(k.threads), args, smem,
                              stream));
     count_launch();
     return TK_OK;
