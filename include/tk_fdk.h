@@ -297,7 +297,7 @@ int tk_bp_select_variant(int i);
  * (FP32 sums without atomics in the box); where that does not apply (row steps
  * below 1/2, very large footprints) lanes on 32 consecutive slices of one voxel
  * column, accumulating each projection's box in two-word fixed point with
- * integer shared atomics (2^-34 or finer of the tile's largest contribution),
+ * integer shared atomics (2^-25 or finer of the tile's largest contribution),
  * or with FP32 atomics when the source lies inside the field of view;
  * 1 lanes on 32 voxel columns, each walking its slices (FP32 shared
  * atomics); 2 the slice-lane form with FP32 shared atomics.  Same weights
