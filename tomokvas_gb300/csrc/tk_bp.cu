@@ -26,6 +26,7 @@
 //  * accumulation is FP32 in registers; each voxel is written once.
 #include "tk_bp_core.cuh"
 #include "tk_common.cuh"
+#include "tk_fp_plan.h"
 #include "tk_internal.h"
 
 #include <cmath>
@@ -1237,13 +1238,12 @@ __global__ void __launch_bounds__(TX *TY, 2)
 // -> this one: 512^3 at scale 1.5 into 360 x 768^2 94.9 -> 72.5 ms; 256^2 x 224
 // at scale 1.2 into 240 x 320 x 272 7.71 -> 5.47 ms; 256^3 at scale 1 into
 // 180 x 256^2 5.63 -> 4.05 ms; 48^2 x 40 into 60 x 64^2 0.331 -> 0.132 ms.
+// (When it is taken, and its shape: tk_fp_plan.h.)
 struct FpRows {
     int TZ;       // slices of a chunk
     int GP;       // voxels of a column in shared memory, padding included (odd)
     int nsplit;   // CTAs that share a tile's projections
 };
-
-constexpr int kFpTX = 16, kFpTY = 8, kFpCols = kFpTX * kFpTY, kFpHalf = kFpCols / 2, kFpWarps = 8, kFpMaxRows = 64;
 
 // Packed FP32 pairs.
 using f32x2 = unsigned long long;
@@ -1984,51 +1984,6 @@ int launch_backproject_quarter(const tk_geometry &g, const void *d_q, int precis
                           compact);
 }
 
-// Shape of a row-lane forward projection (fp_rows_kernel), or K = 0 where it does not apply: the source
-// inside the field of view (U has no bound there), row steps below 1/2 (more than four slices per row), or
-// footprints too large for two CTAs per SM.
-struct FpRowsPlan {
-    int K = 0, TZ = 0, GP = 0, zchunks = 0, BW = 0, BH = 0, stage_elems = 0;
-    size_t smem = 0;
-};
-
-// The box of a 16 x 8 x TZ tile measured from the smallest row and column that its columns inside the field of
-// view reach: columns 0 .. floor(du) + 1 (plus the second tap, plus 3 for the TMA alignment of the origin),
-// rows 0 .. floor(dv) + 2, with du, dv bounded as in bp_box_dims for radii up to W/2.
-static FpRowsPlan fp_rows_plan(const tk_geometry &g, int nz, float zoff)
-{
-    FpRowsPlan p;
-    const double s = std::fabs((double)g.scale), D = g.D;
-    const double ex = s * std::fmax(std::fabs((double)g.cx), std::fabs((double)(g.X - 1) - g.cx));
-    const double ey = s * std::fmax(std::fabs((double)g.cy), std::fabs((double)(g.Y - 1) - g.cy));
-    const double R = std::fmin(0.5 * g.W, std::sqrt(ex * ex + ey * ey) + 1.0);
-    if (!(D - R > 1e-3 * D)) return p;
-    const double dv_min = s * D / (D + R);
-    const int K = dv_min >= 1.0001 ? 2 : dv_min >= 2.0001 / 3.0 ? 3 : dv_min >= 0.50005 ? 4 : 0;
-    if (!K) return p;
-    const double Umax = D / (D - R), dU = D / ((D - R) * (D - R));
-    const double dxy = s * std::sqrt((double)((kFpTX - 1) * (kFpTX - 1) + (kFpTY - 1) * (kFpTY - 1)));
-    const double azmax = s * std::fmax(std::fabs((double)zoff), std::fabs((double)(nz - 1) + zoff));
-    const int BW = (((int)std::floor(dxy * Umax + R * dU * dxy + 0.01) + 6 + 3) / 4 | 1) * 4;  // BW / 4 odd
-    if (BW > 256) return p;
-    auto shape = [&](int TZ) {
-        p.TZ = TZ;
-        p.GP = (TZ + (K == 2 ? 3 : 2 * K)) | 1;
-        p.BW = BW;
-        p.BH = (int)std::floor(s * (TZ - 1) * Umax + azmax * dU * dxy + 0.01) + 3;
-        p.stage_elems = BW * kFpMaxRows;
-        p.smem = kFpWarps * ((size_t)p.stage_elems * 4 + 2 * kFpHalf * sizeof(float4)) + (size_t)kFpCols * p.GP * 4;
-        return p.BH <= kFpMaxRows && p.smem <= 112 * 1024;  // two CTAs per SM
-    };
-    int TZ = std::min(nz, kFpMaxRows);
-    while (TZ >= 1 && !shape(TZ)) --TZ;
-    if (TZ < std::min(nz, 8)) return p;
-    p.zchunks = (nz + TZ - 1) / TZ;
-    shape((nz + p.zchunks - 1) / p.zchunks);  // even chunks
-    p.K = K;
-    return p;
-}
-
 int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, float zoff, float *d_qbar,
                            int accumulate, cudaStream_t stream)
 {
@@ -2046,9 +2001,30 @@ int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, flo
     const BPVariant shape = {nullptr, nullptr, TK_F32, TX, TY, TZ, 2, false, "fp"};
     int BW, BH;
     if (int rc = bp_box_dims(g, nz, zoff, shape.TX, shape.TY, shape.TZ, shape.coef, 4, &BW, &BH)) return rc;
+    const bool cols = g_fp_variant != 1;
+    const double hw = 0.5 * g.W;
+    const bool fixed = g_fp_variant == 0 && (double)g.D > hw;  // else U has no bound: FP32 atomics
+    // Shared memory of the slice-lane and column-lane forms: two staging boxes, an odd-pitch accumulation box (two words
+    // per cell in the fixed-point form), the slice lanes' geometry table, nb footprint origins.
+    const int boxBW = BW, boxBH = BH;
+    auto scatter_smem = [&](int nb) {
+        const size_t acc_elems = (size_t)((boxBH * (boxBW + 1) + 31) & ~31) * (fixed ? 2 : 1);
+        const size_t geo_bytes = cols ? (size_t)(TX * TY / 32) * 32 * sizeof(float4) : 0;
+        return (2 * (size_t)((boxBW * boxBH + 31) / 32 * 32) + acc_elems) * sizeof(float) + geo_bytes +
+               (size_t)nb * sizeof(int2) + 16;
+    };
+    int dev = 0, sms = 0, per_sm = 0;
+    TK_CUDA(cudaGetDevice(&dev));
+    TK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    TK_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     FpRowsPlan rows;
-    if (g_fp_variant == 0) rows = fp_rows_plan(g, nz, zoff);
-    const int boxBW = BW, boxBH = BH;  // of the slice-lane and column-lane forms
+    if (g_fp_variant == 0) {
+        rows = fp_rows_plan(g, nz, zoff);
+        const int nb = std::min(g.N, kMaxParamProj);
+        const bool two = 2 * (scatter_smem(nb) + 1024) <= (size_t)per_sm;  // 1 KB reserved per CTA
+        if (rows.K && !fp_rows_faster(rows, g.X, g.Y, nz, nb, boxBW * boxBH, two, sms))
+            rows = FpRowsPlan();
+    }
     if (rows.K) {
         BW = rows.BW;
         BH = rows.BH;
@@ -2061,10 +2037,10 @@ int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, flo
     TK_CHECK((long long)tilesX * tilesY < (1ll << 31) && zchunks < 65536, TK_ERR_UNSUPPORTED,
              "volume too large for one launch");
     const bool partial = nz < TZ;
-    // Row lanes (variant 0, the default) or, where fp_rows_plan finds no shape, slice lanes with the two-word
-    // fixed-point box; column lanes (1); slice lanes with FP32 shared atomics (2).  The fixed-point box needs a bound on the contributions that
-    // reach one cell of one projection from one tile (a cell takes the voxels whose u lies in a
-    // 2-pixel band and whose v lies in a 2-row band):
+    // Row lanes (variant 0, the default) or, where fp_rows_plan finds no shape or fp_rows_faster says so, slice lanes with
+    // the two-word fixed-point box; column lanes (1); slice lanes with FP32 shared atomics (2).  The fixed-point box needs
+    // a bound on the contributions that reach one cell of one projection from one tile (a cell takes the voxels whose u
+    // lies in a 2-pixel band and whose v lies in a 2-row band):
     //  - the columns whose u falls in a 2-pixel band lie between two rays from the source, a strip
     //    at most w = 2 / (U_min |scale|) voxels wide; a 16 x 16 grid holds at most
     //    16 (floor(sqrt(2) w) + 1) points of such a strip (per grid line, floor(w / max(|cos|,
@@ -2072,9 +2048,6 @@ int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, flo
     //  - per column, the slices whose row falls in a 2-row band, at most floor(2 / dv_min) + 2,
     //    dv_min = |scale| U_min the smallest row step, and at most the 32 slices of a chunk;
     //  with U = D / (D - S), |S| < W/2 inside the FOV: U_min = D / (D + W/2), U_max = D / (D - W/2).
-    const bool cols = g_fp_variant != 1;
-    const double hw = 0.5 * g.W;
-    const bool fixed = g_fp_variant == 0 && (double)g.D > hw;  // else U has no bound: FP32 atomics
     int cbits = 0;
     float u2max = 0.f;
     if (fixed) {
@@ -2144,24 +2117,14 @@ int launch_forward_project(const tk_geometry &g, const float *d_vol, int nz, flo
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         TK_CHECK(cr == CUDA_SUCCESS, TK_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)cr);
-        // odd-pitch accumulation box (two words per cell in the fixed-point form)
-        const size_t acc_elems = (size_t)((boxBH * (boxBW + 1) + 31) & ~31) * (fixed ? 2 : 1);
-        const size_t geo_bytes = cols ? (size_t)(TX * TY / 32) * 32 * sizeof(float4) : 0;  // slice-lane form
-        const size_t smem = (2 * (size_t)((boxBW * boxBH + 31) / 32 * 32) + acc_elems) * sizeof(float) + geo_bytes +
-                            (size_t)nb * sizeof(int2) + 16;
+        const size_t smem = scatter_smem(nb);
         TK_CHECK(smem <= 227 * 1024, TK_ERR_UNSUPPORTED, "forward project: %zu B of shared memory needed", smem);
         const float *vin = d_vol;
         if (rows.K) {
             const void *rfn = rows.K == 2   ? reinterpret_cast<const void *>(&fp_rows_kernel<2>)
                               : rows.K == 3 ? reinterpret_cast<const void *>(&fp_rows_kernel<3>)
                                             : reinterpret_cast<const void *>(&fp_rows_kernel<4>);
-            int dev = 0, sms = 0;
-            TK_CUDA(cudaGetDevice(&dev));
-            TK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            // small volumes: several CTAs per tile, each its share of the projections (at least 4 per warp),
-            // until the chip has about four waves of CTAs
-            const long long ctas = (long long)tilesX * tilesY * zchunks;
-            const int split = (int)std::max(1ll, std::min<long long>((8ll * sms + ctas - 1) / ctas, nb / (4 * kFpWarps)));
+            const int split = fp_rows_split((long long)tilesX * tilesY * zchunks, nb, sms);
             FpRows fr{rows.TZ, rows.GP, split};
             TK_CUDA(cudaFuncSetAttribute(rfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows.smem));
             void *args_fr[] = {&tmap, &P, &vin, &fr};
