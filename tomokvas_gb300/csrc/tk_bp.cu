@@ -1593,6 +1593,7 @@ struct BPVariant {
     int qcap = 0;  // > 0: bp_quad_kernel with staged boxes of up to qcap bytes (needs quad_eligible)
     bool qauto = false;  // a quarter-turn variant the default selection tries, in table order
     bool zsplit = false;  // fewer slices per tile than the format's default: taken for small volumes (same bits)
+    bool wide = false;    // 16 x 16 columns instead of the format's 16 x 8: taken for large footprints (same bits)
 };
 
 
@@ -1628,10 +1629,10 @@ struct BPVariant {
      reinterpret_cast<const void *>(&bp_cimg_kernel<TK_F16, TX, TY, TZ, ST, true, MB, WK>), TK_F16, TX, TY, TZ, ST, \
      true, "cimg_h" #WK "<f16," #TX "," #TY "," #TZ "," #ST ",occ" #MB ">"}
 // 16-bit storage with FP32 interpolation (update_cimg WALK 4)
-#define TK_BP_CIMG_F(P, PN, TX, TY, TZ, ST, MB) \
+#define TK_BP_CIMG_F(P, PN, TX, TY, TZ, ST, MB, WIDE) \
     {reinterpret_cast<const void *>(&bp_cimg_kernel<P, TX, TY, TZ, ST, false, MB, 4>), \
      reinterpret_cast<const void *>(&bp_cimg_kernel<P, TX, TY, TZ, ST, true, MB, 4>), P, TX, TY, TZ, ST, true, \
-     "cimg_f32i<" PN "," #TX "," #TY "," #TZ "," #ST ",occ" #MB ">"}
+     "cimg_f32i<" PN "," #TX "," #TY "," #TZ "," #ST ",occ" #MB ">", 0, false, false, WIDE}
 
 // The first entry of each storage format is its default.  Every default
 // interpolates in FP32 (FP32 geometry, interpolation weights, interpolation and
@@ -1644,9 +1645,9 @@ struct BPVariant {
 static const BPVariant kVariants[] = {
     TK_BP_DIRECT_PK(16, 8, 32, 4, 4, 2, false),
     TK_BP_QUADF(TK_F16, "f16", 6144, 2, true, 8),
-    TK_BP_CIMG_F(TK_F16, "f16", 16, 8, 64, 2, 4),
+    TK_BP_CIMG_F(TK_F16, "f16", 16, 8, 64, 2, 4, false),
     TK_BP_QUADF(TK_BF16, "bf16", 6144, 2, true, 8),
-    TK_BP_CIMG_F(TK_BF16, "bf16", 16, 8, 64, 2, 4),
+    TK_BP_CIMG_F(TK_BF16, "bf16", 16, 8, 64, 2, 4, false),
     TK_BP_CIMG_PK(TK_F32_COEF, "f32c", 16, 16, 64, 2, 2),
     TK_BP_DIRECT(16, 8, 32, 4),
     TK_BP_QUADF(TK_F16, "f16", 8192, 2, true, 16),   // 16 x 16 tiles when a 16 x 8 tile's footprint exceeds 6 KB
@@ -1673,12 +1674,14 @@ static const BPVariant kVariants[] = {
     TK_BP_CIMG_PK(TK_F16, "f16", 16, 16, 48, 3, 2),
     TK_BP_CIMG(TK_F32_COEF, "f32c", 16, 16, 32, 3, 2),
     TK_BP_CIMG(TK_F32_COEF, "f32c", 16, 16, 32, 2, 3),
-    // few slices per tile for small FP32 volumes (z_split)
+    // few slices per tile for small FP32 volumes (pick_direct)
     TK_BP_DIRECT_PK(16, 8, 8, 8, 8, 4, true),
     TK_BP_DIRECT_PK(16, 8, 4, 8, 8, 4, true),
-    // 16 x 16 tiles of the 16-bit general walks for large footprints (wide_twin)
-    TK_BP_CIMG_F(TK_F16, "f16", 16, 16, 64, 2, 2),
-    TK_BP_CIMG_F(TK_BF16, "bf16", 16, 16, 64, 2, 2),
+    // 16 x 16 tiles for large footprints (wide_twin)
+    TK_BP_CIMG_F(TK_F16, "f16", 16, 16, 64, 2, 2, true),
+    TK_BP_CIMG_F(TK_BF16, "bf16", 16, 16, 64, 2, 2, true),
+    {reinterpret_cast<const void *>(&bp_tma_kernel<StoreF32, 16, 16, 32, 4, 2, true, 2>), nullptr, TK_F32, 16, 16, 32, 4,
+     false, "direct_w2<f32,16,16,32,4>", 0, false, false, true},
 };
 
 static int g_variant_override = -1;  // index into kVariants, set by tk_bp_select_variant
@@ -1697,31 +1700,9 @@ static const BPVariant *pick_variant(int precision)
 // The 16 x 16 variant with v's walk, storage and slices per tile (the same arithmetic, so the same bits), or null.
 static const BPVariant *wide_twin(const BPVariant *v)
 {
-    const char *lt = std::strchr(v->name, '<');
-    const size_t np = lt ? (size_t)(lt - v->name) : std::strlen(v->name);
     for (const auto &c : kVariants)
-        if (&c != v && c.precision == v->precision && c.coef == v->coef && !c.qcap && c.TX == 16 && c.TY == 16 &&
-            c.TZ == v->TZ && std::strncmp(c.name, v->name, np) == 0 && c.name[np] == '<')
-            return &c;
+        if (c.wide && c.precision == v->precision && c.TZ == v->TZ) return &c;
     return nullptr;
-}
-
-// The FP32 variant for `columns` tiles per slice layer and nz slices: the default (32 slices per tile), or the same
-// walk with 8 or 4, where tiles of 32 would leave SMs idle or walk slices past the end.  Estimates of the time per 96
-// projections in us from x CTAs per SM, fitted to cubes of 32 to 256 and to slabs: 32 slices max(80, 75 + 27.5 x),
-// 8 slices 42 + 9.4 x, 4 slices 30 + 6.7 x (a step's geometry, wait and barrier cost about three slices).
-// Measured, 32 / 8 / 4 slices: 64^2 x 48 79 / 53 / 47 us, 96^3 127 / 94 / 107, 128^3 169 / 170 / 211, 160^3
-// 252 / 286 / 376, 512^2 x 16 421 / 275 / 361.
-static const BPVariant *z_split(const BPVariant *v, long long columns, int nz, int sms)
-{
-    auto cost = [&](int TZ) {
-        const double x = (double)(columns * ((nz + TZ - 1) / TZ)) / sms;
-        return TZ == 32 ? std::max(80.0, 75.0 + 27.5 * x) : TZ == 8 ? 42.0 + 9.4 * x : 30.0 + 6.7 * x;
-    };
-    const BPVariant *best = v;
-    for (const auto &c : kVariants)
-        if (c.zsplit && c.precision == v->precision && cost(c.TZ) < cost(best->TZ)) best = &c;
-    return best;
 }
 
 // Analytic bound of a tile's footprint extent (see the derivation in the
@@ -1754,6 +1735,59 @@ int bp_box_dims(const tk_geometry &g, int nz, float zoff, int TX, int TY, int TZ
     *BW = bw;
     *BH = bh;
     return TK_OK;
+}
+
+// Staged box and shared memory of a general walk's CTA.
+struct TileShape {
+    int BW = 0, BH = 0;
+    size_t smem = 0;
+    int resident(int per_sm) const { return (int)(per_sm / (smem + 1024)); }  // CTAs per SM (1 KB reserved per CTA)
+};
+static int tile_shape(const tk_geometry &g, int nz, float zoff, const BPVariant &v, TileShape *t)
+{
+    const int ES = (int)entry_size(v.precision);
+    if (int rc = bp_box_dims(g, nz, zoff, v.TX, v.TY, v.TZ, v.coef, v.coef ? (ES >= 16 ? 1 : 16 / ES) : 4, &t->BW, &t->BH))
+        return rc;
+    TK_CHECK(!v.coef || t->BW * ES / 4 <= 256, TK_ERR_UNSUPPORTED, "tile footprint of %d entries too wide", t->BW);
+    const int round = v.coef ? 16 : 64;  // 128-byte aligned stages
+    t->smem = (size_t)v.STAGES * ((t->BW * t->BH + round - 1) / round * round) * ES +
+              (size_t)std::min(g.N, kMaxParamProj) * sizeof(int2) + (size_t)v.STAGES * sizeof(uint64_t) + 16;
+    return TK_OK;
+}
+
+// The FP32-sample variant for a launch: v (16 x 8 tiles of 32 slices), its 16 x 16 twin, or the 16 x 8 walk with 8 or 4
+// slices per tile where tiles of 32 would leave SMs idle or walk slices past the end.  Estimates of the time per 96
+// projections in us from x CTAs per SM, fitted to cubes of 32 to 256 and to slabs: 32 slices max(80, 75 + 27.5 x),
+// 8 slices 42 + 9.4 x, 4 slices 30 + 6.7 x (a step's geometry, wait and barrier cost about three slices).
+// Measured, 32 / 8 / 4 slices: 64^2 x 48 79 / 53 / 47 us, 96^3 127 / 94 / 107, 128^3 169 / 170 / 211, 160^3
+// 252 / 286 / 376, 512^2 x 16 421 / 275 / 361.
+// The estimates assume eight thin CTAs per SM.  Their eight boxes shrink little with the slices where the cone is wide or
+// the slab far from the mid-plane, and the table of footprint origins grows with the projections: with five or four
+// resident they take 1.1 and 1.2 times as long, and they are left out where fewer fit than there are to run (64^2 x 256
+// from 720 at scale 1.2, D = 2 W: one 8-slice CTA per SM 2232 us, 32 slices 881).  16 x 16 tiles where two 16 x 8
+// CTAs or one would fit an SM: 192^2 x 100 from 720 at scale 1.45, D = 2 W 3018 -> 2208 us, 512^2 x 64 from 180 1973 ->
+// 1583.
+static const BPVariant *pick_direct(const BPVariant *v, const TileShape &own, const tk_geometry &g, int nz, float zoff,
+                                    int sms, int per_sm)
+{
+    const long long columns = (long long)((g.X + v->TX - 1) / v->TX) * ((g.Y + v->TY - 1) / v->TY);
+    const BPVariant *best = own.resident(per_sm) <= 2 ? wide_twin(v) : v;
+    double least = std::max(80.0, 75.0 + 27.5 * (double)(columns * ((nz + v->TZ - 1) / v->TZ)) / sms);
+    for (const auto &c : kVariants) {
+        if (!c.zsplit || c.precision != v->precision) continue;
+        const int chunks = (nz + c.TZ - 1) / c.TZ;
+        const double x = (double)(columns * chunks) / sms;
+        TileShape t;
+        if (chunks > 65535 || tile_shape(g, nz, zoff, c, &t) != TK_OK || t.smem > 227 * 1024) continue;
+        const int fit = t.resident(per_sm);
+        if (fit < 4 && fit < x) continue;
+        const double cost = (c.TZ == 8 ? 42.0 + 9.4 * x : 30.0 + 6.7 * x) * (fit >= 6 || fit >= x ? 1.0 : fit == 5 ? 1.1 : 1.2);
+        if (cost < least) {
+            least = cost;
+            best = &c;
+        }
+    }
+    return best;
 }
 
 // The quarter-turn kernel's conditions: a square volume of whole 32-column
@@ -1830,12 +1864,6 @@ static int launch_bp_impl(const tk_geometry &g, const void *d_q, int precision, 
         TK_CHECK(v, TK_ERR_INVALID, "backproject: no general variant for precision %d", precision);
     }
     const bool quad = v->qcap > 0;
-    if (precision == TK_F32 && g_variant_override < 0) {
-        int dev = 0, sms = 0;
-        TK_CUDA(cudaGetDevice(&dev));
-        TK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        v = z_split(v, (long long)((g.X + v->TX - 1) / v->TX) * ((g.Y + v->TY - 1) / v->TY), nz, sms);
-    }
     auto encode = get_encode_fn();
     TK_CHECK(encode, TK_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
 
@@ -1844,33 +1872,29 @@ static int launch_bp_impl(const tk_geometry &g, const void *d_q, int precision, 
     const int align = v->coef ? (ES >= 16 ? 1 : 16 / ES) : 4;
     int BW, BH;
     if (int rc = bp_box_dims(g, nz, zoff, v->TX, v->TY, v->TZ, v->coef, align, &BW, &BH)) return rc;
-    const int nb_max = std::min(g.N, kMaxParamProj);
     if (!quad && g_variant_override < 0 && precision != TK_F32_COEF) {
         // The default tiles are 16 x 8 columns, four CTAs of 128 threads per SM (their barriers join four warps, and
         // the last CTAs are half as long): 256^3 FP32 samples from 96 projections 879 -> 819 us, 512^3 6295 -> 6017;
         // 333^2 x 201 BF16 from 301 at scale 1.1 3239 -> 3151, 500^3 FP16 from 200 13506 -> 13010 (16 x 16, two CTAs of
         // 256).  A 16-bit walk whose boxes do not leave room for four takes 16 x 16 tiles where those keep more warps
         // on an SM (512^3 at scale 1.45: 11325 us against 11479).  What 16 x 16 tiles cannot do is refused.
-        int wBW, wBH;
-        if (int rc = bp_box_dims(g, nz, zoff, 16, 16, v->coef ? 64 : 32, v->coef, align, &wBW, &wBH)) return rc;
-        TK_CHECK(!v->coef || wBW * ES / 4 <= 256, TK_ERR_UNSUPPORTED, "tile footprint of %d entries too wide", wBW);
-        const size_t fixed = (size_t)nb_max * sizeof(int2) + 4 * sizeof(uint64_t) + 16;
-        const size_t wide = v->coef ? 2 * (size_t)((wBW * wBH + 15) / 16 * 16) * ES + fixed
-                                    : 4 * (size_t)((wBW * wBH + 63) / 64 * 64) * ES + fixed;
-        TK_CHECK(wide <= 227 * 1024, TK_ERR_UNSUPPORTED, "backproject: %zu B of shared memory needed", wide);
-        if (v->coef) {
-            int dev = 0, per_sm = 0;
-            TK_CUDA(cudaGetDevice(&dev));
-            TK_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-            const size_t own = 2 * (size_t)((BW * BH + 15) / 16 * 16) * ES + fixed;
-            const size_t warps = 4 * std::min<size_t>(4, per_sm / (own + 1024));  // 1 KB reserved per CTA
-            const BPVariant *w = wide_twin(v);
-            if (w && 8 * std::min<size_t>(2, per_sm / (wide + 1024)) > warps) {
-                v = w;
-                BW = wBW;
-                BH = wBH;
-            }
-        }
+        const BPVariant *w = wide_twin(v);
+        TileShape own, wide;
+        if (int rc = tile_shape(g, nz, zoff, *w, &wide)) return rc;
+        TK_CHECK(wide.smem <= 227 * 1024, TK_ERR_UNSUPPORTED, "backproject: %zu B of shared memory needed", wide.smem);
+        if (int rc = tile_shape(g, nz, zoff, *v, &own)) return rc;
+        int dev = 0, sms = 0, per_sm = 0;
+        TK_CUDA(cudaGetDevice(&dev));
+        TK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        TK_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+        if (precision == TK_F32)
+            v = pick_direct(v, own, g, nz, zoff, sms, per_sm);
+        else if (8 * std::min(2, wide.resident(per_sm)) > 4 * std::min(4, own.resident(per_sm)))
+            v = w;
+        TileShape t;
+        if (int rc = tile_shape(g, nz, zoff, *v, &t)) return rc;
+        BW = t.BW;
+        BH = t.BH;
     }
     BH = std::max(1, BH - g_diag_box_shrink);  // 0 unless a self-check test shrinks the staged box
     TK_CHECK(!v->coef || BW * ES / 4 <= 256, TK_ERR_UNSUPPORTED, "tile footprint of %d entries too wide", BW);
