@@ -59,3 +59,25 @@ def test_large_footprints(cuda, W, N, H, X, nz, D, scale, zoff, cZ, precision):
         _lib.check(L.tk_bp_select_variant(-1))
     assert ran >= 2
     assert device.device_error_flags() == 0
+
+
+@pytest.mark.parametrize("precision", ["f16", "bf16", "f32c"])
+@pytest.mark.parametrize("W,X,nz,D,scale,zoff,flips", [(80, 64, 1, 300.0, 1.0, -3.0, 0), (90, 70, 2, 260.0, 1.2, 10.5, 4),
+                                                       (60, 75, 5, 150.0, 0.7, -40.0, 3), (130, 88, 33, 420.0, 1.3, -16.0, 5),
+                                                       (64, 50, 63, 300.0, 1.0, -31.0, 1)])
+def test_thin_slabs_same_bits(cuda, precision, W, X, nz, D, scale, zoff, flips):
+    """Fewer slices than a chunk, whose staged boxes hold the rows of those slices only, against the first slices of a
+    whole chunk."""
+    import torch
+
+    prec = _lib.PRECISIONS[precision]
+    g = FDKGeometry(W=W, N=17, H=100, cX=(W - 1) / 2, cZ=48.3, dfi=float(np.float32(2 * math.pi / 17)), D=D, tau=0.02,
+                    X=X, Y=X - 5, Z=nz, cx=(X - 1) / 2 + 0.7, cy=(X - 6) / 2, rot=0.05, scale=scale, dirx=flips & 1,
+                    diry=flips >> 1 & 1, dirz=flips >> 2 & 1)
+    x = torch.from_numpy(np.random.default_rng(nz).normal(size=(g.N, g.H, W)).astype(np.float32)).cuda()
+    q, s = device.filter_projections(g, x, layout=_lib.TK_LAYOUT_PROJECTION, precision=prec)
+    thin = device.backproject(g, q, s, prec, nz=nz, zoff=zoff).cpu().numpy()
+    whole = device.backproject(g, q, s, prec, nz=64, zoff=zoff).cpu().numpy()
+    assert np.abs(thin).max() > 0
+    np.testing.assert_array_equal(thin, whole[:nz])
+    assert device.device_error_flags() == 0

@@ -1743,10 +1743,10 @@ struct TileShape {
     size_t smem = 0;
     int resident(int per_sm) const { return (int)(per_sm / (smem + 1024)); }  // CTAs per SM (1 KB reserved per CTA)
 };
-static int tile_shape(const tk_geometry &g, int nz, float zoff, const BPVariant &v, TileShape *t)
+static int tile_shape(const tk_geometry &g, int nz, float zoff, const BPVariant &v, int slices, TileShape *t)
 {
     const int ES = (int)entry_size(v.precision);
-    if (int rc = bp_box_dims(g, nz, zoff, v.TX, v.TY, v.TZ, v.coef, v.coef ? (ES >= 16 ? 1 : 16 / ES) : 4, &t->BW, &t->BH))
+    if (int rc = bp_box_dims(g, nz, zoff, v.TX, v.TY, slices, v.coef, v.coef ? (ES >= 16 ? 1 : 16 / ES) : 4, &t->BW, &t->BH))
         return rc;
     TK_CHECK(!v.coef || t->BW * ES / 4 <= 256, TK_ERR_UNSUPPORTED, "tile footprint of %d entries too wide", t->BW);
     const int round = v.coef ? 16 : 64;  // 128-byte aligned stages
@@ -1778,7 +1778,7 @@ static const BPVariant *pick_direct(const BPVariant *v, const TileShape &own, co
         const int chunks = (nz + c.TZ - 1) / c.TZ;
         const double x = (double)(columns * chunks) / sms;
         TileShape t;
-        if (chunks > 65535 || tile_shape(g, nz, zoff, c, &t) != TK_OK || t.smem > 227 * 1024) continue;
+        if (chunks > 65535 || tile_shape(g, nz, zoff, c, c.TZ, &t) != TK_OK || t.smem > 227 * 1024) continue;
         const int fit = t.resident(per_sm);
         if (fit < 4 && fit < x) continue;
         const double cost = (c.TZ == 8 ? 42.0 + 9.4 * x : 30.0 + 6.7 * x) * (fit >= 6 || fit >= x ? 1.0 : fit == 5 ? 1.1 : 1.2);
@@ -1867,11 +1867,18 @@ static int launch_bp_impl(const tk_geometry &g, const void *d_q, int precision, 
     auto encode = get_encode_fn();
     TK_CHECK(encode, TK_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
 
-    // TMA x-coordinate granularity in entries: 16 bytes
     const int ES = (int)entry_size(precision);
-    const int align = v->coef ? (ES >= 16 ? 1 : 16 / ES) : 4;
-    int BW, BH;
-    if (int rc = bp_box_dims(g, nz, zoff, v->TX, v->TY, v->TZ, v->coef, align, &BW, &BH)) return rc;
+    TileShape shape;  // of the staged box, in full chunks; what these cannot do is refused
+    if (quad) {
+        if (int rc = bp_box_dims(g, nz, zoff, v->TX, v->TY, v->TZ, true, ES >= 16 ? 1 : 16 / ES, &shape.BW, &shape.BH))
+            return rc;
+    } else {
+        if (int rc = tile_shape(g, nz, zoff, *v, v->TZ, &shape)) return rc;
+    }
+    // Coefficient walks of fewer slices than a chunk stage the rows of those only: the rows of 64 slices take longer than
+    // a walk of few (512^2 x 5 from 180 at scale 1: FP16 713 -> 314 us, 401 in 16 x 16 tiles; FP32 coefficients 581 -> 308).
+    const bool partial = v->coef && nz < v->TZ;
+    const auto slices = [&](const BPVariant &c) { return partial ? nz : c.TZ; };
     if (!quad && g_variant_override < 0 && precision != TK_F32_COEF) {
         // The default tiles are 16 x 8 columns, four CTAs of 128 threads per SM (their barriers join four warps, and
         // the last CTAs are half as long): 256^3 FP32 samples from 96 projections 879 -> 819 us, 512^3 6295 -> 6017;
@@ -1879,24 +1886,26 @@ static int launch_bp_impl(const tk_geometry &g, const void *d_q, int precision, 
         // 256).  A 16-bit walk whose boxes do not leave room for four takes 16 x 16 tiles where those keep more warps
         // on an SM (512^3 at scale 1.45: 11325 us against 11479).  What 16 x 16 tiles cannot do is refused.
         const BPVariant *w = wide_twin(v);
-        TileShape own, wide;
-        if (int rc = tile_shape(g, nz, zoff, *w, &wide)) return rc;
+        TileShape wide;
+        if (int rc = tile_shape(g, nz, zoff, *w, w->TZ, &wide)) return rc;
         TK_CHECK(wide.smem <= 227 * 1024, TK_ERR_UNSUPPORTED, "backproject: %zu B of shared memory needed", wide.smem);
-        if (int rc = tile_shape(g, nz, zoff, *v, &own)) return rc;
+        if (int rc = tile_shape(g, nz, zoff, *w, slices(*w), &wide)) return rc;
+        if (int rc = tile_shape(g, nz, zoff, *v, slices(*v), &shape)) return rc;
         int dev = 0, sms = 0, per_sm = 0;
         TK_CUDA(cudaGetDevice(&dev));
         TK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         TK_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
         if (precision == TK_F32)
-            v = pick_direct(v, own, g, nz, zoff, sms, per_sm);
-        else if (8 * std::min(2, wide.resident(per_sm)) > 4 * std::min(4, own.resident(per_sm)))
+            v = pick_direct(v, shape, g, nz, zoff, sms, per_sm);
+        else if (8 * std::min(2, wide.resident(per_sm)) > 4 * std::min(4, shape.resident(per_sm)))
             v = w;
-        TileShape t;
-        if (int rc = tile_shape(g, nz, zoff, *v, &t)) return rc;
-        BW = t.BW;
-        BH = t.BH;
+    } else if (!quad) {
+        TK_CHECK(shape.smem <= 227 * 1024, TK_ERR_UNSUPPORTED, "backproject: %zu B of shared memory needed", shape.smem);
     }
-    BH = std::max(1, BH - g_diag_box_shrink);  // 0 unless a self-check test shrinks the staged box
+    if (!quad)
+        if (int rc = tile_shape(g, nz, zoff, *v, slices(*v), &shape)) return rc;
+    const int BW = shape.BW;
+    const int BH = std::max(1, shape.BH - g_diag_box_shrink);  // 0 unless a self-check test shrinks the staged box
     TK_CHECK(!v->coef || BW * ES / 4 <= 256, TK_ERR_UNSUPPORTED, "tile footprint of %d entries too wide", BW);
 
     TK_CHECK(angle0 >= 0, TK_ERR_INVALID, "backproject: negative first angle index");
@@ -1948,7 +1957,6 @@ static int launch_bp_impl(const tk_geometry &g, const void *d_q, int precision, 
     P.qfs = compact ? P.qlen : g.N / 4;
     TK_CHECK(!compact || (quad && qlen > 0), TK_ERR_INVALID, "backproject: a compact image needs the quarter-turn kernel");
 
-    const bool partial = v->coef && nz < v->TZ;
     const void *fn = partial ? v->fn_partial : v->fn;
     for (int b0 = 0; b0 < g.N; b0 += kMaxParamProj) {
         const int nb = std::min(kMaxParamProj, g.N - b0);
