@@ -189,10 +189,12 @@ __device__ __forceinline__ long long frame_row(const ToepParams &P, long long gr
 }
 
 // PLAIN: rows 16-byte aligned, no dark or flat map (with the general code the producers spill more and 300 frames of
-// 256^2 uint16 take 118 us instead of 108).  The general form copies rows in 8- or 4-byte units where they are only
-// aligned to those, instead of loading sample by sample, and reads a run's maps together: 300 frames of W^2 uint16
-// into FP16, W = 500 648 -> 457 us, 300 260 -> 199; with maps W = 256 234 -> 194, 384 546 -> 450, 512 931 -> 772.
-template <int MODE, bool PLAIN>
+// 256^2 uint16 take 118 us instead of 108).  Otherwise rows aligned to 8 or 4 bytes are copied in such units instead of
+// loaded sample by sample, and with MAPS a run's maps are read together: 300 frames of W^2 uint16 into FP16, W = 500
+// 648 -> 457 us, 300 260 -> 199; with maps W = 256 234 -> 194, 384 546 -> 450, 512 931 -> 772.  Without MAPS the map code
+// is left out: it cost rows of any alignment its registers (390 frames of 201 x 181 uint16, rows aligned to 2 bytes,
+// 193 us with it, 152 without).
+template <int MODE, bool PLAIN, bool MAPS>
 __global__ void __launch_bounds__(kToepThreads, 1) filter_toeplitz_kernel(const __grid_constant__ ToepParams P)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(kToepThreads, 1) filter_toeplitz_kernel(const 
 
     auto preprocess = [&](int r, int j0, float (&v)[8]) {
         const float rt = weight_row_term(P.L, r);
-        if (!PLAIN && has_maps(P.L)) {
+        if constexpr (MAPS) {
             pre8_maps(P.L, r, j0, rt, v);
         } else {
 #pragma unroll
@@ -686,12 +688,13 @@ int launch_filter_toeplitz(const LoadParams &L, const float *Hf, int p, void *d_
     const size_t smem = 1024 + (size_t)P.ncores * 256 + (size_t)P.slots * 2 * P.R * 128 +
                         (size_t)2 * 33 * kToepPitch * 4 + 22 * 8 + 128 + (L.gran ? kToepRawBytes : 0);
     TK_CHECK(smem <= 227 * 1024, TK_ERR_UNSUPPORTED, "filter: Toeplitz form needs %zu B of shared memory", smem);
-    const bool plain = L.gran == 16 && !has_maps(L);
+    const bool maps = has_maps(L), plain = L.gran == 16 && !maps;
     const void *fn = nullptr;
     switch (precision) {
-#define TK_TOEP(MODE)                                                                       \
-    fn = plain ? reinterpret_cast<const void *>(&filter_toeplitz_kernel<MODE, true>)         \
-               : reinterpret_cast<const void *>(&filter_toeplitz_kernel<MODE, false>)
+#define TK_TOEP(MODE)                                                                           \
+    fn = plain  ? reinterpret_cast<const void *>(&filter_toeplitz_kernel<MODE, true, false>)     \
+         : maps ? reinterpret_cast<const void *>(&filter_toeplitz_kernel<MODE, false, true>)     \
+                : reinterpret_cast<const void *>(&filter_toeplitz_kernel<MODE, false, false>)
     case TK_F32: TK_TOEP(TK_F32); break;
     case TK_F16: TK_TOEP(TK_F16); break;
     case TK_BF16: TK_TOEP(TK_BF16); break;
