@@ -654,23 +654,41 @@ __global__ void __launch_bounds__(Fft<LG>::NT, Fft<LG>::MINB) filter_coef_kernel
     }
 }
 
+// max(m, |v|); a NaN sample leaves the bound unchanged.
+__device__ __forceinline__ float bound_of(float m, float v)
+{
+    v = fabsf(v);
+    return v == v ? fmaxf(m, v) : m;
+}
 // max |preprocessed sample| over the whole input, as float bits in *maxbits.
 // Each warp takes whole detector rows (lanes on consecutive columns), so the
 // row's offset is formed once per row rather than by a division per sample.
-// With dark and flat maps eight samples per lane are loaded with their pixels
-// before the first is used: 301 x 389 x 500 uint16 135 -> 124 us.  (Skipping
-// samples that cannot pass the lane's maximum, by two compares, cost more in
-// divergence than the logarithms it saved: 164 us.)
+// With dark and flat maps up to eight samples per lane are loaded with their
+// pixels before the first is used: 301 x 389 x 500 uint16 135 -> 124 us.  Rows
+// of up to 128 samples take runs of four, of up to 64 of two: of eight, most
+// would lie past the row (19392 rows of 33 into FP16, with the filter, 45.1 us
+// with runs of eight, 41.1 so).
+// (Skipping samples that cannot pass the lane's maximum, by two compares, cost
+// more in divergence than the logarithms it saved: 164 us.)
+template <int RUN>
+__device__ __forceinline__ float prescan_maps_row(const LoadParams &L, long long off, int r, float rt, int lane, float m)
+{
+    for (int x0 = lane; x0 < L.W; x0 += 32 * RUN) {
+        float raw[RUN], dk[RUN], fl[RUN];
+#pragma unroll
+        for (int i = 0; i < RUN; ++i) raw[i] = x0 + 32 * i < L.W ? load_raw(L, off, x0 + 32 * i) : 0.f;
+        load_maps<RUN>(L, r, x0, 32, dk, fl);
+#pragma unroll
+        for (int i = 0; i < RUN; ++i)
+            if (x0 + 32 * i < L.W) m = bound_of(m, pre_maps(L, x0 + 32 * i, raw[i], dk[i], fl[i], rt));
+    }
+    return m;
+}
 __global__ void __launch_bounds__(256) prescan_kernel(const __grid_constant__ LoadParams L, long long nrows,
                                                       unsigned *maxbits)
 {
-    constexpr int kRun = 8;
     const bool maps = has_maps(L);
     float m = 0.f;
-    auto bound = [&](float v) {
-        v = fabsf(v);
-        if (v == v) m = fmaxf(m, v);  // NaN input leaves the bound unchanged
-    };
     const int lane = threadIdx.x & 31;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     for (long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; row < nrows; row += nwarps) {
@@ -678,17 +696,11 @@ __global__ void __launch_bounds__(256) prescan_kernel(const __grid_constant__ Lo
         const long long off = in_row_offset(L, row, r);
         const float rt = weight_row_term(L, r);
         if (maps) {
-            for (int x0 = lane; x0 < L.W; x0 += 32 * kRun) {
-                float raw[kRun], dk[kRun], fl[kRun];
-#pragma unroll
-                for (int i = 0; i < kRun; ++i) raw[i] = x0 + 32 * i < L.W ? load_raw(L, off, x0 + 32 * i) : 0.f;
-                load_maps<kRun>(L, r, x0, 32, dk, fl);
-#pragma unroll
-                for (int i = 0; i < kRun; ++i)
-                    if (x0 + 32 * i < L.W) bound(pre_maps(L, x0 + 32 * i, raw[i], dk[i], fl[i], rt));
-            }
+            m = L.W <= 64    ? prescan_maps_row<2>(L, off, r, rt, lane, m)
+                : L.W <= 128 ? prescan_maps_row<4>(L, off, r, rt, lane, m)
+                             : prescan_maps_row<8>(L, off, r, rt, lane, m);
         } else {
-            for (int x = lane; x < L.W; x += 32) bound(pre_scalar(L, x, load_raw(L, off, x), rt));
+            for (int x = lane; x < L.W; x += 32) m = bound_of(m, pre_scalar(L, x, load_raw(L, off, x), rt));
         }
     }
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
