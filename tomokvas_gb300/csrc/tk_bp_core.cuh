@@ -62,8 +62,9 @@ __device__ __forceinline__ float slice_v(float aZ, float U, float cZ) { return f
 // detector cell [r, r+1] x [c, c+1], so an update is one shared load of one
 // entry and
 //   A = Q + fu dU,  B = dV + fu dUV,  acc += U^2 (A + fv B)
-// (16-bit storage: the four values converted to FP32 first, eval_f32; the
-// selectable half-math forms take A and B from one packed HFMA2, eval).
+// (16-bit storage: the four values converted to FP32 first, walk 4 of
+// update_cimg; the selectable half-math forms take A and B from one packed
+// HFMA2, eval).
 // Loads use 32-bit shared
 // addresses (inline PTX) so the address of an update is one IMAD.
 template <int PREC> struct Cimg;
@@ -75,7 +76,6 @@ template <> struct Cimg<TK_F32_COEF> {
         asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q), "=f"(du), "=f"(dv), "=f"(duv) : "r"(addr));
         return make_float2(fmaf(fu, du, q), fmaf(fu, duv, dv));
     }
-    static __device__ __forceinline__ float2 eval_f32(uint32_t addr, float fu) { return eval(addr, fu, float2{}); }
 };
 // The two halves of a 16-bit pair word as FP32 (exact conversions): lo is
 // the half in bits 0-15.
@@ -96,18 +96,6 @@ template <int PREC> __device__ __forceinline__ void unpack_pair(uint32_t w, floa
         hi = f.y;
     }
 }
-// FP32 interpolation of a 16-bit entry {(Q, dV), (dU, dUV)}: the four values
-// converted exactly to FP32, then A = fma(fu, dU, Q), B = fma(fu, dUV, dV) --
-// the operations of the FP32 coefficient format on the stored values.
-template <int PREC> __device__ __forceinline__ float2 eval16_f32(uint32_t addr, float fu)
-{
-    uint32_t lo, hi;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(lo), "=r"(hi) : "r"(addr));
-    float q, dv, du, duv;
-    unpack_pair<PREC>(lo, q, dv);
-    unpack_pair<PREC>(hi, du, duv);
-    return make_float2(fmaf(fu, du, q), fmaf(fu, duv, dv));
-}
 template <> struct Cimg<TK_F16> {
     static constexpr int kBytes = 8, kAlign = 2;
     static __device__ __forceinline__ float2 eval(uint32_t addr, float, float2 fu2raw)
@@ -119,7 +107,6 @@ template <> struct Cimg<TK_F16> {
                                   *reinterpret_cast<const __half2 *>(&lo));
         return __half22float2(h);
     }
-    static __device__ __forceinline__ float2 eval_f32(uint32_t addr, float fu) { return eval16_f32<TK_F16>(addr, fu); }
 };
 template <> struct Cimg<TK_BF16> {
     static constexpr int kBytes = 8, kAlign = 2;
@@ -132,7 +119,6 @@ template <> struct Cimg<TK_BF16> {
                                          *reinterpret_cast<const __nv_bfloat162 *>(&lo));
         return __bfloat1622float2(h);
     }
-    static __device__ __forceinline__ float2 eval_f32(uint32_t addr, float fu) { return eval16_f32<TK_BF16>(addr, fu); }
 };
 
 // fu packed for the 16-bit HFMA2 (carried in the bits of a float2.x).
@@ -320,6 +306,7 @@ template <int PREC, int TZ, bool ALL_IN, bool PARTIAL, int WALK = 0>
 __device__ __forceinline__ void update_cimg(uint32_t sbase, uint32_t row_bytes, float v0, float dv, float fu,
                                             float U2, float Hm1, int zlast, float (&acc)[TZ])
 {
+    static_assert(WALK != 4 || TZ % 2 == 0, "walk 4 takes pairs of slices");
     const float2 fu2 = pack_fu<PREC>(fu);
     if constexpr ((WALK == 2 || WALK == 3) && PREC == TK_F16 && !PARTIAL && (TZ % 2 == 0)) {
         const __half2 fuh = *reinterpret_cast<const __half2 *>(&fu2.x);
@@ -368,7 +355,7 @@ __device__ __forceinline__ void update_cimg(uint32_t sbase, uint32_t row_bytes, 
                            *reinterpret_cast<const uint32_t *>(&fv2), w2, acc[z], acc[z + 1]);
             }
         }
-    } else if constexpr (WALK == 4 && PREC != TK_F32_COEF && (TZ % 2 == 0)) {
+    } else if constexpr (WALK == 4 && PREC != TK_F32_COEF) {
 #pragma unroll
         for (int z = 0; z < TZ; z += 2) {
             if (PARTIAL && z > zlast) break;
@@ -420,7 +407,7 @@ __device__ __forceinline__ void update_cimg(uint32_t sbase, uint32_t row_bytes, 
             const float fl = __fadd_rd(v, kMagic);
             const float fv = v - (fl - kMagic);
             const uint32_t addr = (uint32_t)__float_as_int(fl) * row_bytes + sbase;
-            const float2 ab = WALK == 4 ? Cimg<PREC>::eval_f32(addr, fu) : Cimg<PREC>::eval(addr, fu, fu2);
+            const float2 ab = Cimg<PREC>::eval(addr, fu, fu2);
             const float val = fmaf(fv, ab.y, ab.x);
             if constexpr (ALL_IN) {
                 acc[z] = fmaf(U2, val, acc[z]);

@@ -80,26 +80,6 @@ __device__ __forceinline__ float pre_scalar(const LoadParams &L, int x, float ra
         return pre_finish(L, x, fmaxf(raw - L.dark_v, L.floor_counts) * L.inv_den, rt);
     return L.weight_in ? raw * cosine_weight_rt(L, rt, x) : raw;
 }
-// Either, one sample with its own loads.
-__device__ __forceinline__ float pre_from_raw(const LoadParams &L, int r, int x, float raw, float rt)
-{
-    float val = raw;
-    if (L.input_type == TK_INPUT_U16) {
-        float t;
-        if (L.dark || L.flat) {
-            const size_t px = (size_t)r * L.W + x;
-            const float dk = L.dark ? L.dark[px] : L.dark_v;
-            const float fl = L.flat ? L.flat[px] : L.flat_v;
-            t = __fdividef(fmaxf(raw - dk, L.floor_counts), fmaxf(fl - dk, L.floor_counts));
-        } else {
-            t = fmaxf(raw - L.dark_v, L.floor_counts) * L.inv_den;
-        }
-        val = fmaf(L.A, __logf(t), L.B);
-        if (L.invert) val = -val;
-    }
-    if (!L.weight_in) return val;
-    return val * cosine_weight_rt(L, rt, x);
-}
 // Dark and flat of the pixels x0, x0 + step, ... of row r (N of them, those below W).  A caller loads a run of
 // them before it uses the first: one by one, each sample would wait for its own two loads.
 template <int N>

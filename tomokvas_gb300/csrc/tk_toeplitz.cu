@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kToepThreads, 1) filter_toeplitz_kernel(const 
             pre8_maps(P.L, r, j0, rt, v);
         } else {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = (j0 + e < W) ? pre_from_raw(P.L, r, j0 + e, v[e], rt) : 0.f;
+            for (int e = 0; e < 8; ++e) v[e] = (j0 + e < W) ? pre_scalar(P.L, j0 + e, v[e], rt) : 0.f;
         }
     };
     if (warp < kToepProdWarps && (PLAIN || P.L.gran)) {
