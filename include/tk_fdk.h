@@ -295,8 +295,8 @@ int tk_bp_select_variant(int i);
 /* Forward projector (tk_forward_project / tk_fdk_backward):
  * 0 (default) lanes on detector rows, gathering the slices that reach them
  * (FP32 sums without atomics in the box); where that does not apply (row steps
- * below 1/2, very large footprints) lanes on 32 consecutive slices of one voxel
- * column, accumulating each projection's box in two-word fixed point with
+ * below 1/2, very large footprints) or would be slower (large footprints, few
+ * projections) lanes on 32 consecutive slices of one voxel column, accumulating each projection's box in two-word fixed point with
  * integer shared atomics (2^-25 or finer of the tile's largest contribution),
  * or with FP32 atomics when the source lies inside the field of view;
  * 1 lanes on 32 voxel columns, each walking its slices (FP32 shared

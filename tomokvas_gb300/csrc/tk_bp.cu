@@ -988,7 +988,7 @@ __global__ void __launch_bounds__(TX *TY, 2)
 }
 
 // ---------------------------------------------------------------------------
-// Forward projector with slice lanes (where fp_rows_kernel does not apply; same
+// Forward projector with slice lanes (where fp_rows_kernel does not apply or is slower; same
 // weights, masks, box and drain as fp_scatter_kernel).  Lane l of warp w holds slice z0 + l
 // of the warp's 32 voxel columns (tile rows 2w and 2w+1), and the warp walks
 // its columns one by one.  The lanes of one shared atomic then sit on the
